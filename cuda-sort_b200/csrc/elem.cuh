@@ -100,6 +100,53 @@ __device__ __forceinline__ uint64_t shfl_d(uint64_t v, int d) {
     return __shfl_down_sync(0xffffffffu, (unsigned long long)v, d);
 }
 
+// The value 1, opaque to the compiler (every launch has gridDim.z == 1).  A
+// multiplication by it is a register move on the FMA pipe.
+//
+// Why: a compare-exchange written as a compare and selects runs on the ALU pipe
+// alone, which takes a warp instruction every two cycles: 5 instructions, 10
+// cycles per pair of records (measured in a register-only loop, 8 warps per
+// scheduler), while the FMA pipe idles.  Moving the payloads with predicated
+// multiplications leaves 3 ALU and 3 FMA instructions: 7.0 cycles.  For 64-bit
+// keys the compiler turns compare + selects into a minimum and a maximum with a
+// comparison each, 16 cycles; one comparison with one or both words moved on the
+// FMA pipe takes 9.3 or 12.5, and two of the first to one of the second 8.7.
+__device__ __forceinline__ int opaque_one() {
+    int r;
+    asm("mov.u32 %0, %%nctaid.z;" : "=r"(r));
+    return r;
+}
+
+// PTX of one word's exchange under predicate q (operands by number): on the
+// FMA pipe (ONE: the operand that holds opaque_one()) or by selects.
+#define B200S_SWAP_FMA(A, B, ONE, T) \
+    "mul.lo.u32 " T ", %" A ", %" ONE ";\n\t@q mul.lo.u32 %" A ", %" B ", %" ONE ";\n\t@q mul.lo.u32 %" B ", " T \
+    ", %" ONE ";\n\t"
+#define B200S_SWAP_SEL(A, B, T) \
+    "selp.b32 " T ", %" B ", %" A ", q;\n\tselp.b32 %" B ", %" A ", %" B ", q;\n\tmov.b32 %" A ", " T ";\n\t"
+
+// Ascending compare-exchange of two unsigned 64-bit values (strict): the low
+// words on the FMA pipe, the high words there too when FMA_HIGH.
+template <bool FMA_HIGH>
+__device__ __forceinline__ void cex_u64(uint64_t& lo, uint64_t& hi) {
+    uint32_t a0 = uint32_t(lo), a1 = uint32_t(lo >> 32), b0 = uint32_t(hi), b1 = uint32_t(hi >> 32);
+    const int one = opaque_one();
+    if constexpr (FMA_HIGH)
+        asm("{\n\t.reg .pred q;\n\t.reg .u32 u, w;\n\t.reg .u64 x, y;\n\t"
+            "mov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tsetp.lt.u64 q, y, x;\n\t"
+            B200S_SWAP_FMA("0", "2", "4", "u") B200S_SWAP_FMA("1", "3", "4", "w") "}"
+            : "+r"(a0), "+r"(a1), "+r"(b0), "+r"(b1)
+            : "r"(one));
+    else
+        asm("{\n\t.reg .pred q;\n\t.reg .u32 u, w;\n\t.reg .u64 x, y;\n\t"
+            "mov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tsetp.lt.u64 q, y, x;\n\t"
+            B200S_SWAP_FMA("0", "2", "4", "u") B200S_SWAP_SEL("1", "3", "w") "}"
+            : "+r"(a0), "+r"(a1), "+r"(b0), "+r"(b1)
+            : "r"(one));
+    lo = uint64_t(a1) << 32 | a0;
+    hi = uint64_t(b1) << 32 | b0;
+}
+
 // ---- int32 keys --------------------------------------------------------------
 struct ElemI32 {
     static constexpr bool kKeysOnly = true;  // tie order unobservable
@@ -149,12 +196,13 @@ struct ElemU64 {
     static __device__ __forceinline__ Reg shfl(Reg v, int m) { return shfl_x(v, m); }
     static __device__ __forceinline__ Reg shfl_down(Reg v, int d) { return shfl_d(v, d); }
     static __device__ __forceinline__ bool after(Reg a, Reg b) { return b < a; }
-    static __device__ __forceinline__ void cex(Reg& lo, Reg& hi) {
-        const Reg a = lo, b = hi;
-        const bool sw = b < a;
-        lo = sw ? b : a;
-        hi = sw ? a : b;
+    // Number Q of a layer: one in three moves both words on the FMA pipe,
+    // which balances the two pipes.
+    template <int Q>
+    static __device__ __forceinline__ void cexq(Reg& lo, Reg& hi) {
+        cex_u64<Q % 3 == 0>(lo, hi);
     }
+    static __device__ __forceinline__ void cex(Reg& lo, Reg& hi) { cex_u64<false>(lo, hi); }
     static __device__ __forceinline__ Reg pick(Reg own, Reg other, bool upper) {
         const bool take = upper ? (own < other) : (other < own);
         return take ? other : own;
@@ -179,13 +227,13 @@ struct ElemRecI32 {
     }
     static __device__ __forceinline__ Reg shfl_down(Reg v, int d) { return Reg{shfl_d(v.key, d), shfl_d(v.data, d)}; }
     static __device__ __forceinline__ bool after(const Reg& a, const Reg& b) { return b.key < a.key; }
+    // Strict: ties keep their places.
     static __device__ __forceinline__ void cex(Reg& lo, Reg& hi) {
-        const Reg a = lo, b = hi;
-        const bool sw = b.key < a.key;          // strict: ties keep their places
-        lo.key = sw ? b.key : a.key;
-        lo.data = sw ? b.data : a.data;
-        hi.key = sw ? a.key : b.key;
-        hi.data = sw ? a.data : b.data;
+        asm("{\n\t.reg .pred q;\n\t.reg .s32 t;\n\t.reg .u32 u;\n\t"
+            "setp.lt.s32 q, %1, %0;\n\tmin.s32 t, %0, %1;\n\tmax.s32 %1, %0, %1;\n\tmov.s32 %0, t;\n\t"
+            B200S_SWAP_FMA("2", "3", "4", "u") "}"
+            : "+r"(lo.key), "+r"(hi.key), "+r"(lo.data), "+r"(hi.data)
+            : "r"(opaque_one()));
     }
     static __device__ __forceinline__ Reg pick(Reg own, Reg other, bool upper) {
         const bool take = upper ? (own.key < other.key) : (other.key < own.key);
@@ -238,6 +286,25 @@ struct ElemRecI32S {
     }
 };
 
+// The same order on one 64-bit word per record, the key above the position;
+// the payload stays behind and is fetched by position when the sorted record
+// is written (kGather).  Two words per compare-exchange instead of three, a
+// comparison of one 64-bit value instead of two words with a tie case, and
+// 8 bytes per record through shared memory instead of 12; the words are
+// distinct, so any sorting network gives the stable order.
+struct ElemRecI32G : ElemU64 {
+    using Mem = RecI32;
+    static constexpr bool kStable = true;
+    static constexpr bool kGather = true;
+    static __device__ __forceinline__ Reg from_mem(Mem m, int pos) {
+        return uint64_t(uint32_t(m.key) ^ 0x80000000u) << 32 | uint32_t(pos);
+    }
+    static __device__ __forceinline__ int position(Reg r) { return int(uint32_t(r)); }
+    static __device__ __forceinline__ Mem to_mem(Reg r, int32_t data) {
+        return Mem{int32_t(uint32_t(r >> 32) ^ 0x80000000u), data};
+    }
+};
+
 // ---- records: uint64 key + int32 payload -------------------------------------
 struct alignas(16) RegRecU64 {
     uint64_t key;
@@ -256,16 +323,29 @@ struct ElemRecU64 {
     }
     static __device__ __forceinline__ Reg shfl_down(Reg v, int d) { return Reg{shfl_d(v.key, d), shfl_d(v.data, d)}; }
     static __device__ __forceinline__ bool after(const Reg& a, const Reg& b) { return b.key < a.key; }
-    // Field by field: whole-struct selects of this padded register record
-    // made the compiler spill in the large tiles.
-    static __device__ __forceinline__ void cex(Reg& lo, Reg& hi) {
-        const Reg a = lo, b = hi;
-        const bool sw = b.key < a.key;
-        lo.key = sw ? b.key : a.key;
-        lo.data = sw ? b.data : a.data;
-        hi.key = sw ? a.key : b.key;
-        hi.data = sw ? a.data : b.data;
+    // Word by word (whole-struct selects of this padded register record made
+    // the compiler spill), the words shared between the pipes: even numbers of
+    // a layer move one word on the FMA pipe, odd ones two.
+    template <int Q>
+    static __device__ __forceinline__ void cexq(Reg& lo, Reg& hi) {
+        uint32_t a0 = uint32_t(lo.key), a1 = uint32_t(lo.key >> 32), b0 = uint32_t(hi.key), b1 = uint32_t(hi.key >> 32);
+        const int one = opaque_one();
+        if constexpr (Q % 2 == 0)
+            asm("{\n\t.reg .pred q;\n\t.reg .u32 u, w, z;\n\t.reg .u64 x, y;\n\t"
+                "mov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tsetp.lt.u64 q, y, x;\n\t"
+                B200S_SWAP_FMA("0", "2", "6", "u") B200S_SWAP_SEL("1", "3", "w") B200S_SWAP_SEL("4", "5", "z") "}"
+                : "+r"(a0), "+r"(a1), "+r"(b0), "+r"(b1), "+r"(lo.data), "+r"(hi.data)
+                : "r"(one));
+        else
+            asm("{\n\t.reg .pred q;\n\t.reg .u32 u, w, z;\n\t.reg .u64 x, y;\n\t"
+                "mov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tsetp.lt.u64 q, y, x;\n\t"
+                B200S_SWAP_FMA("0", "2", "6", "u") B200S_SWAP_SEL("1", "3", "w") B200S_SWAP_FMA("4", "5", "6", "z") "}"
+                : "+r"(a0), "+r"(a1), "+r"(b0), "+r"(b1), "+r"(lo.data), "+r"(hi.data)
+                : "r"(one));
+        lo.key = uint64_t(a1) << 32 | a0;
+        hi.key = uint64_t(b1) << 32 | b0;
     }
+    static __device__ __forceinline__ void cex(Reg& lo, Reg& hi) { cexq<0>(lo, hi); }
     static __device__ __forceinline__ Reg pick(Reg own, Reg other, bool upper) {
         const bool take = upper ? (own.key < other.key) : (other.key < own.key);
         Reg r;
@@ -298,15 +378,19 @@ struct ElemRecU64S {
         return a.key < b.key || (a.key == b.key && a.pos < b.pos);
     }
     static __device__ __forceinline__ bool after(const Reg& a, const Reg& b) { return lt(b, a); }
+    // b < a as one 96-bit subtraction of (key, position), its borrow the
+    // exchange; two of the four words move on the FMA pipe.
     static __device__ __forceinline__ void cex(Reg& lo, Reg& hi) {
-        const Reg a = lo, b = hi;
-        const bool sw = lt(b, a);
-        lo.key = sw ? b.key : a.key;
-        lo.data = sw ? b.data : a.data;
-        lo.pos = sw ? b.pos : a.pos;
-        hi.key = sw ? a.key : b.key;
-        hi.data = sw ? a.data : b.data;
-        hi.pos = sw ? a.pos : b.pos;
+        uint32_t a0 = uint32_t(lo.key), a1 = uint32_t(lo.key >> 32), b0 = uint32_t(hi.key), b1 = uint32_t(hi.key >> 32);
+        asm("{\n\t.reg .pred q;\n\t.reg .u32 d, u, w, y, z;\n\t"
+            "sub.cc.u32 d, %7, %6;\n\tsubc.cc.u32 d, %2, %0;\n\tsubc.cc.u32 d, %3, %1;\n\tsubc.u32 d, 0, 0;\n\t"
+            "setp.ne.u32 q, d, 0;\n\t"
+            B200S_SWAP_FMA("0", "2", "8", "u") B200S_SWAP_SEL("1", "3", "w") B200S_SWAP_FMA("4", "5", "8", "y")
+            B200S_SWAP_SEL("6", "7", "z") "}"
+            : "+r"(a0), "+r"(a1), "+r"(b0), "+r"(b1), "+r"(lo.data), "+r"(hi.data), "+r"(lo.pos), "+r"(hi.pos)
+            : "r"(opaque_one()));
+        lo.key = uint64_t(a1) << 32 | a0;
+        hi.key = uint64_t(b1) << 32 | b0;
     }
     static __device__ __forceinline__ Reg pick(Reg own, Reg other, bool upper) {
         const bool take = upper ? lt(own, other) : lt(other, own);

@@ -47,26 +47,24 @@
 
 namespace b200s {
 
-// Compare-exchange number Q of a layer.  An element type with kFmaSplit runs
-// two of every three in its cex_fma form, which leaves the minimum on the ALU
-// pipe and forms the maximum as a + b - min with two integer multiply-adds on
-// the FMA pipe (exact in two's complement), so both pipes share the layer.
+// Compare-exchange number Q of a layer: element types with cexq share a
+// layer's exchanges between the ALU and the FMA pipe by that number.
 template <class E, class = void>
-struct fma_split : std::false_type {};
+struct has_cexq : std::false_type {};
 template <class E>
-struct fma_split<E, std::void_t<decltype(E::kFmaSplit)>> : std::integral_constant<bool, E::kFmaSplit> {};
-
-template <class E, class = void>
-struct fma_period : std::integral_constant<int, 3> {};
-template <class E>
-struct fma_period<E, std::void_t<decltype(E::kFmaPeriod)>> : std::integral_constant<int, E::kFmaPeriod> {};
+struct has_cexq<E, std::void_t<decltype(&E::template cexq<0>)>> : std::true_type {};
 
 template <class E, int Q>
 __device__ __forceinline__ void xcex(typename E::Reg& lo, typename E::Reg& hi) {
-    constexpr int P = fma_period<E>::value;  // P > 0: one in P in the FMA form; P < 0: all but one in -P
-    if constexpr (fma_split<E>::value && (P > 0 ? (Q % P) == 0 : (Q % -P) != 0)) E::cex_fma(lo, hi);
+    if constexpr (has_cexq<E>::value) E::template cexq<Q>(lo, hi);
     else E::cex(lo, hi);
 }
+
+// Element types that leave the payload out of the network (see ElemRecI32G).
+template <class E, class = void>
+struct gathers : std::false_type {};
+template <class E>
+struct gathers<E, std::void_t<decltype(E::kGather)>> : std::integral_constant<bool, E::kGather> {};
 
 // Streaming (evict-first) global accesses of one element of each memory
 // layout; records move as one 8- or 16-byte access, so their arrays must be
@@ -84,6 +82,27 @@ __device__ __forceinline__ void xp_stcs(uint64_t* p, uint64_t v) {
     __stcs(reinterpret_cast<unsigned long long*>(p), (unsigned long long)v);
 }
 __device__ __forceinline__ void xp_stcs(RecI32* p, RecI32 v) { __stcs(reinterpret_cast<int2*>(p), make_int2(v.key, v.data)); }
+
+// 16-byte records (their buffers are 16-byte aligned).
+__device__ __forceinline__ RecU64 xp_ldcs(const RecU64* p) {
+    RecU64 m;
+    from_u4<0>(__ldcs(reinterpret_cast<const uint4*>(p)), m);
+    return m;
+}
+__device__ __forceinline__ void xp_stcs(RecU64* p, const RecU64& v) {
+    uint4 u;
+    to_u4<0>(u, v);
+    __stcs(reinterpret_cast<uint4*>(p), u);
+}
+// Records in a buffer that is only 4-byte aligned.
+template <class M>
+__device__ __forceinline__ M load_narrow(const M* p) {
+    return *p;
+}
+template <class M>
+__device__ __forceinline__ void store_narrow(M* p, const M& v) {
+    *p = v;
+}
 
 // Element types whose tie order cannot be observed (keys alone: equal keys
 // are indistinguishable) may sort a thread's registers with any network that
