@@ -14,18 +14,25 @@ namespace b200s {
 template <class E, int LK, int LW, int MINB = 1>
 struct PackedXc {
     using S = Shape<LK, 5, LW>;
-    static_assert(LW > 0, "multi-warp tiles");
     static constexpr int CTA = S::TPA;
-    static constexpr size_t SMEM = size_t(xc_smem_elems<LK, S::LOGW>()) * sizeof(typename E::Reg);
+    static constexpr size_t SMEM = xc_smem_bytes<E, LK, S::LOGW>();
+    template <bool CHECK>
+    static cudaError_t launch_form(const void* in, void* out, int n, long long arrays, cudaStream_t st) {
+        static std::atomic<unsigned long long> done{0};
+        auto fn = k_sort_packed_xc<E, S, MINB, CHECK>;
+        cudaError_t e = opt_in_smem<SMEM>(reinterpret_cast<const void*>(fn), done);
+        const auto* src = static_cast<const typename E::Mem*>(in);
+        auto* dst = static_cast<typename E::Mem*>(out);
+        for (long long first = 0; e == cudaSuccess && first < arrays; first += 0x7fffffffLL) {
+            const long long grid = arrays - first < 0x7fffffffLL ? arrays - first : 0x7fffffffLL;
+            e = launch_pdl(fn, unsigned(grid), CTA, SMEM, st, src + first * n, dst + first * n, n);
+        }
+        return e;
+    }
     static cudaError_t launch(const void* in, void* out, int n, long long arrays, long long,
                               cudaStream_t st, unsigned opts) {
-        static std::atomic<unsigned long long> done{0};
-        auto fn = k_sort_packed_xc<E, S, MINB>;
-        cudaError_t e = opt_in_smem<SMEM>(reinterpret_cast<const void*>(fn), done);
-        if (e != cudaSuccess) return e;
-        const long long grid = arrays < 0x7fffffffLL ? arrays : 0x7fffffffLL;
-        return launch_pdl(fn, unsigned(grid), CTA, SMEM, st, static_cast<const typename E::Mem*>(in),
-                          static_cast<typename E::Mem*>(out), n, arrays, opts);
+        return (opts & kOptSortedCheck) ? launch_form<true>(in, out, n, arrays, st)
+                                        : launch_form<false>(in, out, n, arrays, st);
     }
     static cudaError_t launch_list(const void* in, void* out, const int* off, const int* ids, int count,
                                    cudaStream_t st) {
@@ -79,7 +86,7 @@ struct ClusterXcKernel {
 template <class E, int LK, int LG, int LW, int LC, bool SB, int MINB = 1>
 struct ClusterXc {
     using Tile = ClusterTile<E, LK, LG, LW, LC, SB, MINB, ClusterXcKernel,
-                             size_t(xc_smem_elems<LK, LK + LG + LW>())>;
+                             size_t(xc_smem_elems<E, LK, LK + LG + LW>())>;
     // Attach to the registered cluster entry of the same shape, CTAs per
     // array and dtype (whose element type may be another of the same
     // records, e.g. a compact form).

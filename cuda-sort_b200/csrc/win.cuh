@@ -1,0 +1,265 @@
+// The reflection network of one tile with every layer in registers: the layers
+// are cut into windows across stage boundaries (win_layout.h), one trip through
+// shared memory each.  Used by the kernels of cta_xpose.cuh.
+//
+// The comparators are those of cusort_v6.hpp:90-142 in the same order, with
+// the keep-own rule of cusort.hpp:460-472, so the output, tie order of records
+// included, is the reference's.  Keys alone (kKeysOnly) sort each thread's
+// registers with Batcher's odd-even merge sort instead of stages 0 .. LK-1.
+//
+// What bounds it: at 16 elements per thread the shared-memory pipe (83 % of its
+// wavefronts at W = 4096 records) with the issue slots close behind (74 %);
+// the ALU and FMA pipes share the compare-exchanges (63 % each, elem.cuh).
+// 32 records per thread take a quarter fewer trips but their unrolled code
+// (100 KB and more) overflows the instruction cache: W = 1024 / 4096 / 8192 in
+// 41.6 / 57.7 / 73.0 us per 4 M records against 38.9 / 51.5 / 66.5 with 16.
+#pragma once
+#include "win_layout.h"
+#include "xpose.cuh"
+
+namespace b200s {
+
+// Lanes of one bank sweep: 2^m elements of this register type fill the banks.
+template <class R>
+constexpr int win_m() {
+    return sizeof(R) == 16 ? 3 : sizeof(R) == 8 ? 4 : 5;
+}
+
+template <class E, int LK, int LOGW>
+struct Win {
+    using R = typename E::Reg;
+    using P = WinPlan<LK, LOGW, win_m<R>()>;
+    static constexpr int K = 1 << LK, LT = P::LT, LW = P::LW;
+    static constexpr int kElems = P::kT.elems;  // shared-memory elements of the tile
+    static constexpr int kWindows = P::kT.windows, kMerges = P::kT.merges;
+
+    // Layouts by number: 0 .. kWindows the windows (0 natural), kIo the
+    // coalesced global one, kMerge + i the windows of a whole-tile merge.
+    static constexpr int kIo = -1, kMerge = 100;
+    static constexpr WinLayout layout(int l) {
+        return l == kIo ? P::kT.io : l >= kMerge ? P::kT.merge[l - kMerge] : P::kT.win[l];
+    }
+
+    // Address part of thread t in a layout (MIR: the thread bits below the
+    // reflection's stage complemented).
+    template <int L, bool MIR>
+    static __device__ __forceinline__ int base(const int t) {
+        constexpr WinLayout w = layout(L);
+        int a = 0;
+        sfor<0, LT>([&](auto jc) {
+            constexpr int j = decltype(jc)::value;
+            constexpr int wt = P::kT.weight[w.thr[j]];
+            constexpr bool flip = MIR && w.thr[j] < w.st;
+            const int bit = (t >> j) & 1;
+            a += (flip ? 1 - bit : bit) * wt;
+        });
+        return a;
+    }
+    template <int L>
+    static __device__ __forceinline__ void put(const R (&v)[K], const int t, R* sm) {
+        constexpr WinLayout w = layout(L);
+        const int bp = base<L, false>(t);
+        int bm = bp;
+        if constexpr (w.refl >= 0) bm = base<L, true>(t);
+        sfor<0, K>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            constexpr int off = P::reg_off(w, q);
+            sh_st(&sm[(P::mirrored(w, q) ? bm : bp) + off], v[q]);
+        });
+    }
+    template <int L>
+    static __device__ __forceinline__ void get(R (&v)[K], const int t, const R* sm) {
+        constexpr WinLayout w = layout(L);
+        const int bp = base<L, false>(t);
+        int bm = bp;
+        if constexpr (w.refl >= 0) bm = base<L, true>(t);
+        sfor<0, K>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            constexpr int off = P::reg_off(w, q);
+            v[q] = sh_ld(&sm[(P::mirrored(w, q) ? bm : bp) + off]);
+        });
+    }
+    // Warps of padding.  In a layout where every warp holds its natural part
+    // of the tile (32 * K consecutive elements), a warp whose part starts at or
+    // beyond n holds only padding, which never moves (keep-own rule): it skips
+    // the layout's layers, and its trips, since the places at and beyond n hold
+    // padding from the load on.  `dead` is uniform over the warp.
+    static constexpr bool own_part(int l) { return LW > 0 && P::same_warps(layout(l), layout(0)); }
+    static __device__ __forceinline__ bool dead(const int t, const int n) {
+        return LW > 0 && ((t >> 5) << (LK + 5)) >= n;
+    }
+
+    // One trip.  A thread puts its elements exactly where it got them, so no
+    // thread's put can touch a place that another has still to read, and one
+    // barrier between the puts and the next gets is enough: a warp's while
+    // every warp keeps its part of the tile, else the team's.
+    template <int A, int B, class Bar>
+    static __device__ __forceinline__ void move(R (&v)[K], const int t, R* sm, const bool skip, const Bar& bar) {
+        constexpr bool local = P::same_warps(layout(A), layout(B));
+        if (!own_part(A) || !skip) put<A>(v, t, sm);
+        if constexpr (local) __syncwarp();
+        else bar();
+        if (!own_part(B) || !skip) get<B>(v, t, sm);
+    }
+    template <int L>
+    static __device__ __forceinline__ void layers(R (&v)[K]) {
+        constexpr WinLayout w = layout(L);
+        sfor<0, w.layers>([&](auto ic) {
+            constexpr int r = w.layers - 1 - decltype(ic)::value;
+            sfor<0, K>([&](auto qc) {
+                constexpr int q = decltype(qc)::value;
+                constexpr int p = r == w.refl ? (q ^ (K - 1)) : (q | (1 << r));
+                if constexpr (!(q & (1 << r))) xcex<E, q>(v[q], v[p]);
+            });
+        });
+    }
+    // One window: the trip from layout A and layout B's layers.
+    template <int A, int B, class Bar>
+    static __device__ __forceinline__ void window(R (&v)[K], const int t, R* sm, const bool skip, const Bar& bar) {
+        if constexpr (own_part(A) && own_part(B)) {
+            if (!skip) {
+                put<A>(v, t, sm);
+                __syncwarp();
+                get<B>(v, t, sm);
+                layers<B>(v);
+            }
+        } else {
+            move<A, B>(v, t, sm, skip, bar);
+            if (!own_part(B) || !skip) layers<B>(v);
+        }
+    }
+    // The network, from and to the natural layout; n: elements that are not
+    // padding.
+    template <class Bar>
+    static __device__ __forceinline__ void network(R (&v)[K], const int t, const int n, R* sm, const Bar& bar) {
+        const bool skip = dead(t, n);
+        if (!skip) {
+            if constexpr (keys_only<E>::value) xp_reg_sort_oem<E, LK>(v);
+            else sfor<0, LK>([&](auto sc) { xp_reg_stage<E, LK, decltype(sc)::value>(v); });
+        }
+        sfor<1, kWindows + 1>([&](auto wc) {
+            constexpr int L = decltype(wc)::value;
+            window<L - 1, L>(v, t, sm, skip, bar);
+        });
+    }
+    // The merges on bits LOGW-1 .. 0, from layout kMerge to the natural one.
+    template <class Bar>
+    static __device__ __forceinline__ void merge(R (&v)[K], const int t, const int n, R* sm, const Bar& bar) {
+        const bool skip = dead(t, n);
+        layers<kMerge>(v);
+        sfor<1, kMerges>([&](auto mc) {
+            constexpr int L = kMerge + decltype(mc)::value;
+            window<L - 1, L>(v, t, sm, skip, bar);
+        });
+        if constexpr (P::kT.merge[kMerges - 1].reg[0] != 0) move<kMerge + kMerges - 1, 0>(v, t, sm, skip, bar);
+    }
+
+    // ---- global memory ------------------------------------------------------
+    // Each warp moves its natural part of the tile (32 * K consecutive
+    // elements) with coalesced accesses through the region, in the layout kIo,
+    // so that only the warp has to synchronise.  `first`: index of the tile's
+    // element 0 in the array of n; elements at or beyond n are padding.
+    // A record buffer that is only 4-byte aligned moves word by word.
+    static __device__ __forceinline__ bool wide(const void* p) {
+        return (reinterpret_cast<uintptr_t>(p) & (sizeof(typename E::Mem) == 8 ? 7u : 3u)) == 0;
+    }
+    static __device__ __forceinline__ typename E::Mem load_one(const typename E::Mem* p, const bool w) {
+        if (w) return xp_ldcs(p);
+        return load_narrow(p);
+    }
+    static __device__ __forceinline__ int io_index(const int t) { return (t & 31) | ((t >> 5) << (LK + 5)); }
+
+    // Load into the natural layout.  pay: the payloads by position (gathered types).
+    static __device__ __forceinline__ void load(R (&v)[K], const typename E::Mem* src, const int t, const int first,
+                                                const int n, R* sm, int32_t* pay = nullptr) {
+        const int i0 = io_index(t), b = base<kIo, false>(t);
+        const bool w = wide(src);
+        if constexpr (E::kStable && sizeof(R) == 16) {
+            // four-word registers: the loads first, as they come from memory
+            // (built into registers one by one they were waited for one by
+            // one: 127 -> 100 us at W = 1024)
+            typename E::Mem m[K];
+            sfor<0, K>([&](auto qc) {
+                constexpr int q = decltype(qc)::value;
+                const int idx = first + i0 + 32 * q;
+                if (idx < n) m[q] = load_one(src + idx, w);
+            });
+            sfor<0, K>([&](auto qc) {
+                constexpr int q = decltype(qc)::value;
+                constexpr int off = P::reg_off(P::kT.io, q);
+                const int idx = first + i0 + 32 * q;
+                sh_st(&sm[b + off], idx < n ? E::from_mem(m[q], idx) : E::pad());
+            });
+        } else {
+            sfor<0, K>([&](auto qc) {
+                constexpr int q = decltype(qc)::value;
+                const int i = i0 + 32 * q, idx = first + i;
+                v[q] = E::pad();
+                if (idx < n) {
+                    const typename E::Mem m = load_one(src + idx, w);
+                    v[q] = E::from_mem(m, idx);
+                    if constexpr (gathers<E>::value)
+                        if (pay) pay[i] = m.data;
+                }
+            });
+            sfor<0, K>([&](auto qc) {
+                constexpr int q = decltype(qc)::value;
+                constexpr int off = P::reg_off(P::kT.io, q);
+                sh_st(&sm[b + off], v[q]);
+            });
+        }
+        __syncwarp();
+        get<0>(v, t, sm);
+    }
+    // Store from the natural layout.
+    static __device__ __forceinline__ void store(const R (&v)[K], typename E::Mem* dst, const int t, const int first,
+                                                 const int n, R* sm) {
+        if (dead(t, n - first)) return;
+        put<0>(v, t, sm);
+        __syncwarp();
+        const int i0 = io_index(t), b = base<kIo, false>(t);
+        const bool w = wide(dst);
+        sfor<0, K>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            constexpr int off = P::reg_off(P::kT.io, q);
+            const int idx = first + i0 + 32 * q;
+            const R x = sh_ld(&sm[b + off]);
+            if (idx < n) {
+                if (w) xp_stcs(dst + idx, E::to_mem(x));
+                else store_narrow(dst + idx, E::to_mem(x));
+            }
+        });
+    }
+    // The same for gathered types: every payload is fetched (from pay when
+    // set, else from src, the unsorted array) before `ready` lets any thread
+    // store, because src may be dst.
+    template <class Ready>
+    static __device__ __forceinline__ void store_gather(const R (&v)[K], const typename E::Mem* src,
+                                                        typename E::Mem* dst, const int t, const int first,
+                                                        const int n, R* sm, const int32_t* pay, const Ready& ready) {
+        put<0>(v, t, sm);
+        __syncwarp();
+        const int i0 = io_index(t), b = base<kIo, false>(t);
+        typename E::Mem m[K];
+        sfor<0, K>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            constexpr int off = P::reg_off(P::kT.io, q);
+            const R x = sh_ld(&sm[b + off]);
+            int32_t d = 0;
+            if (first + i0 + 32 * q < n) d = pay ? pay[E::position(x)] : src[E::position(x)].data;
+            m[q] = E::to_mem(x, d);
+        });
+        ready();
+        const bool w = wide(dst);
+        sfor<0, K>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            const int idx = first + i0 + 32 * q;
+            if (idx < n) {
+                if (w) xp_stcs(dst + idx, m[q]);
+                else store_narrow(dst + idx, m[q]);
+            }
+        });
+    }
+};
+
+}  // namespace b200s

@@ -12,9 +12,9 @@ void register_xc_cluster_rec(std::vector<KernelEntry>& o) {
     ClusterXc<ElemRecI32, 4, 5, 4, 1, false>::attach_to(o, 1);
     ClusterXc<ElemRecI32, 4, 5, 4, 2, false>::attach_to(o, 1);
     ClusterXc<ElemRecI32, 4, 5, 4, 3, false>::attach_to(o, 1);
-    ClusterXc<ElemRecI32S, 4, 5, 5, 0, true>::attach_to(o, 1);
-    ClusterXc<ElemRecI32S, 4, 5, 5, 1, true>::attach_to(o, 1);
-    ClusterXc<ElemRecI32S, 4, 5, 5, 2, true>::attach_to(o, 1);
+    ClusterXc<ElemRecI32G, 4, 5, 5, 0, true>::attach_to(o, 1);
+    ClusterXc<ElemRecI32G, 4, 5, 5, 1, true>::attach_to(o, 1);
+    ClusterXc<ElemRecI32G, 4, 5, 5, 2, true>::attach_to(o, 1);
 }
 
 }  // namespace b200s
