@@ -86,21 +86,19 @@ __device__ __forceinline__ void xc_cluster_network(typename E::Reg (&v)[1 << LK]
     }
 }
 
-// One array in one CTA: load, network, store.  CHECK: with the sortedness test.
-template <class E, class S, bool CHECK>
+// One array by a team of S::TPA threads (bar: its barrier): load, network,
+// store.  CHECK: with the sortedness test (the team is the CTA).
+template <class E, class S, bool CHECK, class Bar = CtaBarrier>
 __device__ __forceinline__ void xc_sort_array(const typename E::Mem* src, typename E::Mem* dst, const int n,
-                                              const int t, typename E::Reg* sm) {
+                                              const int t, typename E::Reg* sm, const Bar& bar = Bar()) {
     using R = typename E::Reg;
     using W = Win<E, S::LK, S::LOGW>;
     R v[S::K];
     int32_t* pay = gathers<E>::value ? reinterpret_cast<int32_t*>(sm + W::kElems) : nullptr;
     W::load(v, src, t, 0, n, sm, pay);
     bool skip = false;
-    if constexpr (CHECK) {
-        __syncthreads();  // the test's scratch lies in the region
-        skip = team_in_order<E, S>(v, t, sm);
-    }
-    if (!skip) W::network(v, t, n, sm, CtaBarrier{});
+    if constexpr (CHECK) skip = W::in_order(v, t, sm);
+    if (!skip) W::network(v, t, n, sm, bar);
     if (skip && src == dst) return;
     if constexpr (gathers<E>::value) W::store_gather(v, src, dst, t, 0, n, sm, pay, [] {});
     else W::store(v, dst, t, 0, n, sm);

@@ -259,25 +259,23 @@ struct ClusterTile {
     }
 };
 
-// The persistent ragged kernel of element type E.
-template <class E, int CTA, int NB, int LKA, int LKB, bool SB = false, int MINB = 1>
+// The persistent ragged kernel of element type E (EW: the type of its windowed
+// buckets).
+template <class E, class EW, int CTA, int NB, int LKA, int LKB, int MINB>
 struct Ragged {
-    static constexpr size_t SMEM = ragged_smem<E, CTA, NB, LKA, LKB, SB>();
+    static constexpr size_t SMEM = ragged_smem<E, EW, CTA, NB>();
+    static constexpr auto kernel() { return k_sort_ragged<E, EW, CTA, NB, LKA, LKB, MINB>; }
     static cudaError_t launch(const void* in, void* out, const int* off, const int* ids, RaggedCtl* ctl,
                               unsigned family_mask, unsigned dedicated_mask, int grid, cudaStream_t st) {
-        auto fn = k_sort_ragged<E, CTA, NB, LKA, LKB, SB, MINB>;
-        if (SMEM > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fn),
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM));
-            if (e != cudaSuccess) return e;
-        }
-        fn<<<dim3(unsigned(grid)), dim3(CTA), SMEM, st>>>(static_cast<const typename E::Mem*>(in),
-                                                          static_cast<typename E::Mem*>(out), off, ids, ctl,
-                                                          family_mask, dedicated_mask);
-        return cudaGetLastError();
+        static std::atomic<unsigned long long> done{0};
+        auto fn = kernel();
+        cudaError_t e = opt_in_smem<SMEM>(reinterpret_cast<const void*>(fn), done);
+        if (e != cudaSuccess) return e;
+        return launch_pdl(fn, unsigned(grid), CTA, SMEM, st, static_cast<const typename E::Mem*>(in),
+                          static_cast<typename E::Mem*>(out), off, ids, ctl, family_mask, dedicated_mask);
     }
     static int resident_per_sm() {
-        auto fn = k_sort_ragged<E, CTA, NB, LKA, LKB, SB, MINB>;
+        auto fn = kernel();
         if (SMEM > 48 * 1024 &&
             cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(SMEM)) != cudaSuccess)

@@ -35,6 +35,8 @@ unsigned ragged_dedicated_mask(int dtype, int stable);
 void dedicated_entries(int dtype, int stable, int nb, unsigned* mask, int* idx, bool* xc);
 bool cluster_xc(int dtype, int stable, int entry);
 int lookup_default_entry(int dtype, int stable, long long n, int* persistent);
+cudaError_t launch_binning(const int* off, int arrays, RaggedCtl* ctl, int* ids, int* oids, const BinSpec& spec,
+                           int max_grid, cudaStream_t st);
 
 namespace {
 
@@ -121,15 +123,8 @@ extern "C" b200s_status b200s_sort_ragged_noalloc(b200s_dtype dtype, uint32_t fl
 
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     const int n = int(arrays);
-    // The counters are shared with every other call: start them at zero.
-    e = cudaMemsetAsync(&s->ctl, 0, sizeof(RaggedCtl), cs);
-    if (e != cudaSuccess) return cuda_error(e, "scratch reset");
-    const int bin_threads = 256;
-    const int bin_grid = std::max(1, std::min(sms * 4, (n + bin_threads - 1) / bin_threads));
-    k_bin_count<<<bin_grid, bin_threads, 0, cs>>>(d_offsets, n, &s->ctl, spec);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "bin count launch");
-    k_bin_scatter<<<bin_grid, bin_threads, 0, cs>>>(d_offsets, n, &s->ctl, s->ids, s->oids, spec);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "bin scatter launch");
+    e = launch_binning(d_offsets, n, &s->ctl, s->ids, s->oids, spec, sms * 4, cs);
+    if (e != cudaSuccess) return cuda_error(e, "ragged binning");
     // the plan's routing: buckets with their own launch run after the
     // persistent kernel on the same stream (no side streams here); the tile
     // table that sets it loads on the first lookup

@@ -19,6 +19,7 @@ b200s_status cuda_error(cudaError_t e, const char* what);
 int effective_stable(int dtype, uint32_t flags);
 int ceil_log2(long long n);
 int lookup_default_entry(int dtype, int stable, long long n, int* persistent);
+int narrow_alternative(int idx, long long arrays);
 b200s_status launch_packed(int idx, int persistent, const void* in, void* out, int n, long long arrays,
                            cudaStream_t st, unsigned opts = 0);
 
@@ -27,7 +28,9 @@ const std::vector<RaggedEntry>& ragged_registry() {
         std::vector<RaggedEntry> v;
         register_ragged_i32(v);
         register_ragged_rec(v);
+        register_ragged_rec_stable(v);
         register_ragged_u64(v);
+        register_ragged_u64rec(v);
         return v;
     }();
     return all;
@@ -76,6 +79,32 @@ unsigned ragged_dedicated_mask(int dtype, int stable) {
     return g_dedicated_mask[dtype][stable];
 }
 
+// Resets the control block and bins the arrays (see ragged.cuh): one launch
+// with programmatic stream serialization up to kBinSmall arrays.
+cudaError_t launch_binning(const int* off, int arrays, RaggedCtl* ctl, int* ids, int* oids, const BinSpec& spec,
+                           int max_grid, cudaStream_t st) {
+    if (arrays <= kBinSmall) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1);
+        cfg.blockDim = dim3(1024);
+        cfg.stream = st;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k_bin_small, off, arrays, ctl, ids, oids, spec);
+    }
+    cudaError_t e = cudaMemsetAsync(ctl, 0, sizeof(RaggedCtl), st);
+    if (e != cudaSuccess) return e;
+    const int threads = 256;
+    const int grid = std::max(1, std::min(max_grid, (arrays + threads - 1) / threads));
+    k_bin_count<<<grid, threads, 0, st>>>(off, arrays, ctl, spec);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    k_bin_scatter<<<grid, threads, 0, st>>>(off, arrays, ctl, ids, oids, spec);
+    return cudaGetLastError();
+}
+
 // Registry entries of the dedicated buckets (bit b of `mask`: bucket b, W =
 // 2^(kRaggedLmin + b)): the tabled single-CTA tile of that working length.
 // Buckets without one (none tabled, or a cluster tile) stay in the persistent
@@ -122,6 +151,32 @@ bool cluster_xc(int dtype, int stable, int entry) {
     return lookup_default_entry(dtype, stable, 1LL << k.log2w, &form) >= 0 && form == 3;
 }
 
+// One pass over the offsets (see b200s_internal_check_offsets).  One block
+// writes the flag itself; more add to a word that the caller has cleared.
+constexpr int kCheckThreads = 1024;
+template <class T>
+__global__ void __launch_bounds__(kCheckThreads) k_check_offsets(const T* off, long long arrays, long long total,
+                                                                 int longest, int* off32, int* flag) {
+    bool bad = false;
+    for (long long i = (long long)blockIdx.x * kCheckThreads + threadIdx.x; i <= arrays;
+         i += (long long)gridDim.x * kCheckThreads) {
+        const long long o = off[i];
+        if (i == 0) bad |= o != 0;
+        if (i == arrays) {
+            bad |= o != total;
+        } else {
+            const long long n = (long long)off[i + 1] - o;
+            bad |= n < 0 || n > longest;
+        }
+        if (off32) off32[i] = int(o);
+    }
+    bad = __syncthreads_or(bad) != 0;
+    if (threadIdx.x == 0) {
+        if (gridDim.x == 1) *flag = bad;
+        else if (bad) atomicOr(flag, 1);
+    }
+}
+
 }  // namespace b200s
 
 using namespace b200s;
@@ -150,12 +205,21 @@ struct b200s_plan {
     cudaStream_t capture = nullptr;
     cudaStream_t side[kSides] = {};  // cluster and dedicated buckets run beside the persistent kernel
     cudaEvent_t fork = nullptr, join[kSides] = {};
-    // the graph of the last (in, out, offsets, arrays)
+    cudaEvent_t done = nullptr;           // end of the last call: calls on another stream wait for it
+    cudaStream_t last_stream = nullptr;
+    bool used = false;
+    // The buffers and array count of a call; the graph's and the last call's.
+    struct Call {
+        const void* in = nullptr;
+        void* out = nullptr;
+        const int* off = nullptr;
+        long long arrays = -1;
+        bool operator==(const Call& c) const {
+            return in == c.in && out == c.out && off == c.off && arrays == c.arrays;
+        }
+    };
     cudaGraphExec_t exec = nullptr;
-    const void* g_in = nullptr;
-    void* g_out = nullptr;
-    const int* g_off = nullptr;
-    long long g_arrays = -1;
+    Call graph_call, last_call;
     // plain per-length launches: ids grouped by exact length on the host
     int* plain_ids = nullptr;
     struct Group {
@@ -169,16 +233,14 @@ namespace {
 // present / over_present: bit b set when bucket b (cluster class i) may hold
 // an array; classes with a launch of their own are skipped when their bit is
 // clear (all ones: launch everything, as a graph must).
+// over_count: arrays of each cluster class when the caller knows them (null:
+// not known); a class of a few arrays then takes the latency tile that a
+// packed batch of as many arrays would (narrow_alternative).
 b200s_status record_sequence(b200s_plan* p, const void* in, void* out, const int* off, int arrays,
-                             cudaStream_t st, uint32_t present = ~0u, uint32_t over_present = ~0u) {
-    cudaError_t e = cudaMemsetAsync(p->ctl, 0, sizeof(RaggedCtl), st);
-    if (e != cudaSuccess) return cuda_error(e, "ragged control reset");
-    const int bin_threads = 256;
-    const int bin_grid = std::max(1, std::min(p->bin_grid, (arrays + bin_threads - 1) / bin_threads));
-    k_bin_count<<<bin_grid, bin_threads, 0, st>>>(off, arrays, p->ctl, p->spec);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "bin count launch");
-    k_bin_scatter<<<bin_grid, bin_threads, 0, st>>>(off, arrays, p->ctl, p->ids, p->oids, p->spec);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "bin scatter launch");
+                             cudaStream_t st, uint32_t present = ~0u, uint32_t over_present = ~0u,
+                             const int* over_count = nullptr) {
+    cudaError_t e = launch_binning(off, arrays, p->ctl, p->ids, p->oids, p->spec, p->bin_grid, st);
+    if (e != cudaSuccess) return cuda_error(e, "ragged binning");
     // Fork: the cluster buckets and the dedicated buckets run on side streams
     // (largest first, round robin) while the persistent kernel runs on st;
     // join before returning.
@@ -196,10 +258,11 @@ b200s_status record_sequence(b200s_plan* p, const void* in, void* out, const int
     int k = 0;
     for (int i = p->spec.n_over - 1; i >= 0; --i) {
         if (!((over_present >> i) & 1u)) continue;
-        const KernelEntry& ke = registry()[size_t(p->over_entry[i])];
+        const int entry = over_count ? narrow_alternative(p->over_entry[i], over_count[i]) : p->over_entry[i];
+        const KernelEntry& ke = registry()[size_t(entry)];
         cudaStream_t ss = side_stream(k++);
         if (!ss) return cuda_error(e, "fork");
-        e = (p->over_xc[i] ? ke.launch_cluster_list_xc : ke.launch_cluster_list)(
+        e = (p->over_xc[i] && ke.launch_cluster_list_xc ? ke.launch_cluster_list_xc : ke.launch_cluster_list)(
             in, out, off, p->oids + size_t(i) * p->spec.stride, &p->ctl->ocount[i], max_count, ss);
         if (e != cudaSuccess) return cuda_error(e, "cluster bucket launch");
     }
@@ -222,6 +285,41 @@ b200s_status record_sequence(b200s_plan* p, const void* in, void* out, const int
         if ((e = cudaStreamWaitEvent(st, p->join[s], 0)) != cudaSuccess) return cuda_error(e, "join wait");
     }
     return B200S_OK;
+}
+
+// Calls share the plan's scratch: one on another stream than the last waits
+// for that one's end.  (Inside a stream capture the order is the caller's.)
+b200s_status begin_call(b200s_plan* p, cudaStream_t st, bool capturing) {
+    if (p->used && p->last_stream != st && !capturing) {
+        const cudaError_t e = cudaStreamWaitEvent(st, p->done, 0);
+        if (e != cudaSuccess) return cuda_error(e, "plan order");
+    }
+    return B200S_OK;
+}
+b200s_status end_call(b200s_plan* p, cudaStream_t st, bool capturing) {
+    if (capturing) return B200S_OK;
+    const cudaError_t e = cudaEventRecord(p->done, st);
+    if (e != cudaSuccess) return cuda_error(e, "plan order");
+    p->last_stream = st;
+    p->used = true;
+    return B200S_OK;
+}
+b200s_status is_capturing(cudaStream_t st, bool* out) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(st, &c);
+    if (e != cudaSuccess) return cuda_error(e, "stream capture status");
+    *out = c != cudaStreamCaptureStatusNone;
+    return B200S_OK;
+}
+
+// The sequence launched straight into st.
+b200s_status run_direct(b200s_plan* p, const void* in, void* out, const int* off, int arrays, cudaStream_t st,
+                        bool capturing, uint32_t present = ~0u, uint32_t over_present = ~0u,
+                        const int* over_count = nullptr) {
+    b200s_status s = begin_call(p, st, capturing);
+    if (s == B200S_OK) s = record_sequence(p, in, out, off, arrays, st, present, over_present, over_count);
+    if (s == B200S_OK) s = end_call(p, st, capturing);
+    return s;
 }
 
 }  // namespace
@@ -315,6 +413,7 @@ b200s_status b200s_plan_create(b200s_plan** out, b200s_dtype dtype, uint32_t fla
     p->oids = p->plain_ids + stride;
     e = cudaStreamCreateWithFlags(&p->capture, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming);
     for (int s = 0; s < b200s_plan::kSides && e == cudaSuccess; ++s) {
         e = cudaStreamCreateWithFlags(&p->side[s], cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->join[s], cudaEventDisableTiming);
@@ -339,6 +438,7 @@ b200s_status b200s_plan_destroy(b200s_plan* p) {
         if (p->join[s]) cudaEventDestroy(p->join[s]);
     }
     if (p->fork) cudaEventDestroy(p->fork);
+    if (p->done) cudaEventDestroy(p->done);
     if (p->scratch) cudaFree(p->scratch);
     delete p;
     return B200S_OK;
@@ -354,8 +454,19 @@ b200s_status b200s_sort_ragged(b200s_plan* p, const void* d_in, void* d_out, con
     cudaError_t e = cudaSetDevice(p->device);
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (p->flags & B200S_PLAN_NO_GRAPH) return record_sequence(p, d_in, d_out, d_offsets, int(arrays), st);
-    if (!p->exec || p->g_in != d_in || p->g_out != d_out || p->g_off != d_offsets || p->g_arrays != arrays) {
+    bool capturing = false;
+    b200s_status status = is_capturing(st, &capturing);
+    if (status != B200S_OK) return status;
+    // A graph serves calls that repeat the previous call's buffers.  Other
+    // calls launch the sequence directly: a capture and instantiation per call
+    // took about 450 us of host time with a wait for the device, the direct
+    // launches about 20.  A stream that is being captured takes them too.
+    const b200s_plan::Call call{d_in, d_out, d_offsets, arrays};
+    const bool repeated = call == p->last_call;
+    p->last_call = call;
+    if ((p->flags & B200S_PLAN_NO_GRAPH) || capturing || !(repeated || (p->exec && call == p->graph_call)))
+        return run_direct(p, d_in, d_out, d_offsets, int(arrays), st, capturing);
+    if (!p->exec || !(call == p->graph_call)) {
         if (p->exec) {
             // the previous graph may still run on another stream
             cudaDeviceSynchronize();
@@ -378,14 +489,12 @@ b200s_status b200s_sort_ragged(b200s_plan* p, const void* d_in, void* d_out, con
             p->exec = nullptr;
             return cuda_error(e, "graph instantiate");
         }
-        p->g_in = d_in;
-        p->g_out = d_out;
-        p->g_off = d_offsets;
-        p->g_arrays = arrays;
+        p->graph_call = call;
     }
+    if ((status = begin_call(p, st, false)) != B200S_OK) return status;
     e = cudaGraphLaunch(p->exec, st);
     if (e != cudaSuccess) return cuda_error(e, "graph launch");
-    return B200S_OK;
+    return end_call(p, st, false);
 }
 
 b200s_status b200s_sort_ragged_hinted(b200s_plan* p, const void* d_in, void* d_out, const int32_t* d_offsets,
@@ -399,18 +508,26 @@ b200s_status b200s_sort_ragged_hinted(b200s_plan* p, const void* d_in, void* d_o
     if (!d_in || !d_out || !d_offsets) return set_error(B200S_ERR_INVALID_ARGUMENT, "null buffer");
     // the classes the batch holds, by the binning kernel's rule
     uint32_t present = 0, over_present = 0;
+    int over_count[kMaxOverflow] = {};
     for (int64_t a = 0; a < arrays; ++a) {
         const int n = h_offsets[a + 1] - h_offsets[a];
         if (n <= 0) continue;
         const int l = n <= 1 ? 0 : 32 - __builtin_clz(unsigned(n - 1));
         const int b = (l > kRaggedLmin ? l : kRaggedLmin) - kRaggedLmin;
         if (b < p->spec.nb) present |= 1u << b;
-        else if (l - p->spec.over_lo < p->spec.n_over) over_present |= 1u << (l - p->spec.over_lo);
+        else if (l - p->spec.over_lo < p->spec.n_over) {
+            over_present |= 1u << (l - p->spec.over_lo);
+            ++over_count[l - p->spec.over_lo];
+        }
     }
     cudaError_t e = cudaSetDevice(p->device);
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
-    return record_sequence(p, d_in, d_out, d_offsets, int(arrays), static_cast<cudaStream_t>(stream), present,
-                           over_present);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    bool capturing = false;
+    const b200s_status status = is_capturing(st, &capturing);
+    if (status != B200S_OK) return status;
+    return run_direct(p, d_in, d_out, d_offsets, int(arrays), st, capturing, present, over_present,
+                      over_count);
 }
 
 b200s_status b200s_plan_too_long(b200s_plan* p, void* stream, int64_t* count) {
@@ -479,6 +596,29 @@ b200s_status prepare_plain(b200s_plan* p, const int32_t* h_offsets, int64_t arra
 }  // namespace
 
 extern "C" {
+
+// For the PyTorch operator (not part of the C header): whether offsets (int32,
+// or int64 when is64) start at 0, end at total, never decrease and hold no
+// array longer than longest, as one flag word on the device (0: they do);
+// int64 offsets are copied to off32.
+b200s_status b200s_internal_check_offsets(const void* off, int32_t is64, int64_t arrays, int64_t total,
+                                          int32_t longest, int32_t* off32, int32_t* d_flag, void* stream) {
+    if (!off || !d_flag || arrays < 0 || (is64 && !off32))
+        return set_error(B200S_ERR_INVALID_ARGUMENT, "b200s_internal_check_offsets: bad argument");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const long long blocks = std::min<long long>((arrays + kCheckThreads) / kCheckThreads, 592);
+    cudaError_t e = blocks > 1 ? cudaMemsetAsync(d_flag, 0, sizeof(int32_t), st) : cudaSuccess;
+    if (e == cudaSuccess) {
+        if (is64)
+            k_check_offsets<<<unsigned(blocks), kCheckThreads, 0, st>>>(static_cast<const int64_t*>(off), arrays, total,
+                                                                       longest, off32, d_flag);
+        else
+            k_check_offsets<<<unsigned(blocks), kCheckThreads, 0, st>>>(static_cast<const int*>(off), arrays, total,
+                                                                       longest, nullptr, d_flag);
+        e = cudaGetLastError();
+    }
+    return e == cudaSuccess ? B200S_OK : cuda_error(e, "offset check");
+}
 
 b200s_status b200s_plan_prepare_plain(b200s_plan* p, const int32_t* h_offsets, int64_t arrays) {
     return prepare_plain(p, h_offsets, arrays, false);

@@ -4,13 +4,14 @@
 // launch sequence of a plan is
 //   1. reset the control block (counters, queue head),
 //   2. k_bin_count   - histogram of arrays per working-length bucket,
-//   3. k_bin_scatter - array ids grouped by bucket, largest bucket first,
+//   3. k_bin_scatter - array ids grouped by bucket, largest bucket first
+//                      (up to kBinSmall arrays: 1-3 in one launch, k_bin_small),
 //   4. k_sort_ragged - persistent CTAs pull tasks from a device queue (one
 //                      atomicAdd per task; no waiting on other CTAs).  A task
 //                      is one CTA's worth of arrays of one bucket: the CTA
 //                      splits into teams of TPA threads, one array per team,
-//                      each team running the bitonic network of its bucket's
-//                      tile (multi-warp teams synchronise on a named barrier).
+//                      each team running the network of its bucket's tile
+//                      (multi-warp teams synchronise on a named barrier).
 // Tasks are ordered largest working length first, so the longest tasks start
 // early and the short ones fill the tail.  The bitonic network's cost depends
 // only on the working length, so all teams of a task finish together.
@@ -22,13 +23,14 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include "network.cuh"
+#include "cta_xpose.cuh"
 
 namespace b200s {
 
 constexpr int kMaxBuckets = 16;
 constexpr int kMaxOverflow = 4;
 constexpr int kRaggedLmin = 3;  // smallest bucket: W = 8
+constexpr int kBinSmall = 4096; // arrays of the largest batch that one CTA bins
 
 struct RaggedCtl {
     int count[kMaxBuckets];    // arrays per bucket
@@ -79,6 +81,62 @@ __global__ void k_bin_count(const int* __restrict__ off, int arrays, RaggedCtl* 
     if (threadIdx.x == 0 && over) atomicAdd(&ctl->too_long, over);
 }
 
+// The whole binning of a batch of at most kBinSmall arrays in one CTA: reset,
+// histogram, positions and lists, with the arrays' buckets kept in registers
+// between the two halves.  One launch of about 3 us where the reset and the
+// two kernels below take three launches in a row; from several thousand
+// arrays on one CTA's loads and list stores take longer than that.
+__global__ void __launch_bounds__(1024) k_bin_small(const int* __restrict__ off, int arrays, RaggedCtl* ctl, int* ids,
+                                                    int* oids, BinSpec spec) {
+    constexpr int kPer = kBinSmall / 1024, kClasses = kMaxBuckets + kMaxOverflow;
+    __shared__ int h[kClasses + 1], base[kMaxBuckets];  // h[kClasses]: too long for every kernel
+    const int t = int(threadIdx.x), lane = t & 31;
+    if (t <= kClasses) h[t] = 0;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __syncthreads();
+    int cls[kPer], pos[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int a = i * 1024 + t;
+        const int n = a < arrays ? off[a + 1] - off[a] : 0;
+        int c = -1;
+        if (n > 0) {
+            const int b = bucket_of(n, kRaggedLmin), o = ceil_log2_dev(n) - spec.over_lo;
+            c = b < spec.nb ? b : o < spec.n_over ? kMaxBuckets + o : kClasses;
+        }
+        // one shared atomic per class and warp
+        const unsigned same = __match_any_sync(0xffffffffu, c);
+        int first = 0;
+        if (c >= 0 && lane == __ffs(int(same)) - 1) first = atomicAdd(&h[c], __popc(same));
+        first = __shfl_sync(0xffffffffu, first, __ffs(int(same)) - 1);
+        cls[i] = c;
+        pos[i] = first + __popc(same & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    if (t < kMaxBuckets) {
+        int s = 0;  // larger buckets come first
+        for (int b = t + 1; b < spec.nb; ++b) s += h[b];
+        base[t] = s;
+        ctl->count[t] = h[t];
+        ctl->cursor[t] = 0;
+        ctl->base[t] = s;
+        ctl->dhead[t] = 0;
+    } else if (t < kClasses) {
+        ctl->ocount[t - kMaxBuckets] = h[t];
+    } else if (t == kClasses) {
+        ctl->head = 0;
+        ctl->too_long = h[kClasses];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int c = cls[i], a = i * 1024 + t;
+        if (c >= 0 && c < kMaxBuckets) ids[base[c] + pos[i]] = a;
+        else if (c >= kMaxBuckets && c < kClasses) oids[size_t(c - kMaxBuckets) * spec.stride + pos[i]] = a;
+    }
+}
+
 // ids[] receives array ids grouped by bucket, largest working length first;
 // arrays for the cluster kernels go to their own lists.
 __global__ void k_bin_scatter(const int* __restrict__ off, int arrays, RaggedCtl* ctl, int* ids, int* oids,
@@ -122,6 +180,8 @@ __global__ void k_bin_scatter(const int* __restrict__ off, int arrays, RaggedCtl
     }
 }
 #else
+__global__ void k_bin_small(const int* __restrict__ off, int arrays, RaggedCtl* ctl, int* ids, int* oids,
+                            BinSpec spec);
 __global__ void k_bin_count(const int* __restrict__ off, int arrays, RaggedCtl* ctl, BinSpec spec);
 __global__ void k_bin_scatter(const int* __restrict__ off, int arrays, RaggedCtl* ctl, int* ids, int* oids,
                               BinSpec spec);
@@ -148,79 +208,118 @@ struct FamilyShape {
     using type = Shape<LK, LG, LW>;
 };
 
-template <class E, class S, int CTA, bool SB>
+// Shared-memory bytes of one team of windowed bucket L, a multiple of 16.
+template <class EW, int LK, int L>
+constexpr size_t team_bytes() {
+    return (xc_smem_bytes<EW, LK, L>() + 15) / 16 * 16;
+}
+
+// How the persistent kernel sorts bucket L of element type E (EW: the type
+// its windowed network runs on, ElemRecI32G for stable records):
+//   kWindows   teams of whole warps, the windowed network of win.cuh,
+//   kXpose     several arrays per warp, the one-warp transposed network,
+//   kBlocked   shuffles and registers (network.cuh), one of two families.
+// The first two are the tiles the same lengths take in a packed batch; 16-byte
+// records have no one-warp transposed tile, and int32 arrays below 256 and
+// others below 64 are faster in the blocked form.
+enum RaggedKind { kBlocked, kXpose, kWindows };
+template <class EW>
+constexpr int ragged_lk() {
+    return sizeof(typename EW::Reg) == 4 ? 5 : 4;
+}
+template <class E, class EW>
+constexpr RaggedKind ragged_kind(int L) {
+    if (L >= ragged_lk<EW>() + 5) return kWindows;
+    if (sizeof(typename E::Reg) != 16 && L >= (sizeof(typename E::Reg) == 4 ? 8 : 6)) return kXpose;
+    return kBlocked;
+}
+// log2 threads per array of bucket L.
+template <class E, class EW>
+constexpr int ragged_log_tpa(int L, int family_k, int log_cta) {
+    return L - (ragged_kind<E, EW>(L) == kBlocked ? family_lk(L, family_k, log_cta) : ragged_lk<EW>());
+}
+
+template <class E, class EW, int L, int LKF, int CTA>
 __device__ __forceinline__ void ragged_task(const typename E::Mem* in, typename E::Mem* out,
                                             const int* __restrict__ off, const int* __restrict__ ids,
-                                            int first_id, int count, int local_task,
-                                            unsigned char* smem_raw) {
-    using R = typename E::Reg;
-    static_assert(CTA % S::TPA == 0, "whole teams per CTA");
-    constexpr int APT = CTA / S::TPA;
-    const int team = int(threadIdx.x) / S::TPA;
-    const int t = int(threadIdx.x) % S::TPA;
+                                            const int count, const int local_task, unsigned char* smem_raw) {
+    constexpr int LOGTPA = ragged_log_tpa<E, EW>(L, LKF, log2_const(CTA)), TPA = 1 << LOGTPA;
+    static_assert(TPA <= CTA, "a team fits the CTA");
+    constexpr int APT = CTA / TPA;
+    const int tid = thread_index();
+    const int team = tid >> LOGTPA, t = tid & (TPA - 1);
     const int idx = local_task * APT + team;
     int na = 0;
     long long start = 0;
     if (idx < count) {
-        const int a = ids[first_id + idx];
+        const int a = ids[idx];
         start = off[a];
         na = off[a + 1] - off[a];
     }
-    R* cur = reinterpret_cast<R*>(smem_raw) + size_t(team) * (SB ? 1 : 2) * S::W;
-    R* nxt = SB ? cur : cur + S::W;
-    R v[S::K];
-    load_tile<E, S::K>(v, in + start, t * S::K, na);
-    if constexpr (S::LW > 0) {
-        static_assert(CTA / S::TPA <= 15, "named barrier ids");
-        if constexpr (SB) network<E, S>(v, t, cur, nxt, TeamBarrierSingle{1 + team, S::TPA}, na);
-        else network<E, S>(v, t, cur, nxt, TeamBarrier{1 + team, S::TPA}, na);
+    if constexpr (ragged_kind<E, EW>(L) == kWindows) {
+        static_assert(TPA == 32 || APT <= 15, "named barrier ids");
+        using S = Shape<ragged_lk<EW>(), 5, LOGTPA - 5>;
+        auto* sm = reinterpret_cast<typename EW::Reg*>(smem_raw + size_t(team) * team_bytes<EW, S::LK, L>());
+        xc_sort_array<EW, S, false>(in + start, out + start, na, t, sm, TeamBarrier{1 + team, TPA});
+    } else if constexpr (ragged_kind<E, EW>(L) == kXpose) {
+        constexpr int LK = ragged_lk<EW>(), LG = L - LK;
+        auto* sm = reinterpret_cast<typename E::Reg*>(smem_raw) + team * xp_region<LK, LG>();
+        xp_sort_array<E, LK, LG, keys_only<E>::value ? kXpIoStriped : kXpIoStaged>(in + start, out + start, na, t, sm);
     } else {
+        using R = typename E::Reg;
+        using S = typename FamilyShape<LKF, L, CTA>::type;
+        static_assert(S::LW == 0, "blocked buckets are below a warp");
+        R* cur = reinterpret_cast<R*>(smem_raw);
+        R* nxt = cur;
+        R v[S::K];
+        load_tile<E, S::K>(v, in + start, t * S::K, na);
         network<E, S>(v, t, cur, nxt, CtaBarrier{}, na);
+        store_tile<E, S::K>(v, out + start, t * S::K, na);
     }
-    store_tile<E, S::K>(v, out + start, t * S::K, na);
 }
 
-// NB buckets (W = 8 .. 8 << (NB-1)); bucket b uses family B (K = 2^LKB)
-// when bit b of family_mask is set, else family A (K = 2^LKA); buckets whose
-// bit is set in dedicated_mask are left to their own launches (their ids stay
-// in the list at ctl->base[b]).  SB: one shared-memory buffer per team (two
-// barriers per shared-memory layer, half the shared memory); MINB: CTAs per
-// SM the register budget is sized for.
-template <class E, int CTA, int NB, int LKA, int LKB, bool SB, int MINB>
+// NB buckets (W = 8 .. 8 << (NB-1)); a blocked bucket b uses family B (K =
+// 2^LKB) when bit b of family_mask is set, else family A (K = 2^LKA); buckets
+// whose bit is set in dedicated_mask are left to their own launches (their ids
+// stay in the list at ctl->base[b]).  MINB: CTAs per SM the register budget is
+// sized for.  A CTA's first task is its own number; the further ones come
+// from the queue, each drawn while the previous task is sorted.
+template <class E, class EW, int CTA, int NB, int LKA, int LKB, int MINB>
 __global__ void __launch_bounds__(CTA, MINB) k_sort_ragged(const typename E::Mem* in, typename E::Mem* out,
                                                         const int* __restrict__ off,
                                                         const int* __restrict__ ids, RaggedCtl* ctl,
                                                         unsigned family_mask, unsigned dedicated_mask) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_first[NB], s_tasks[NB], s_base[NB], s_count[NB];
-    __shared__ int s_total, s_task;
+    __shared__ int s_total, s_next[2];
+    // launched with programmatic stream serialization behind the binning kernel
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (threadIdx.x < NB) {
+        const int b = int(threadIdx.x), L = b + kRaggedLmin;
+        const int c = ctl->count[b];
+        const int log_apt = log2_const(CTA) -
+                            ragged_log_tpa<E, EW>(L, ((family_mask >> b) & 1u) ? LKB : LKA, log2_const(CTA));
+        s_tasks[b] = ((dedicated_mask >> b) & 1u) ? 0 : (c + (1 << log_apt) - 1) >> log_apt;
+        s_count[b] = c;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
         int task = 0, base = 0;
         for (int b = NB - 1; b >= 0; --b) {
             // dedicated buckets get no tasks here, but their ids still occupy
             // the list, so the bases count them
-            const int c = ctl->count[b];
-            const int L = b + kRaggedLmin;
-            const int lk = family_lk(L, ((family_mask >> b) & 1u) ? LKB : LKA, log2_const(CTA));
-            const int tpa = 1 << (L - lk);
-            const int apt = CTA / tpa;
             s_first[b] = task;
-            s_tasks[b] = ((dedicated_mask >> b) & 1u) ? 0 : (c + apt - 1) / apt;
             s_base[b] = base;
-            s_count[b] = c;
             task += s_tasks[b];
-            base += c;
+            base += s_count[b];
         }
         s_total = task;
     }
     __syncthreads();
     const int total = s_total;
-    for (;;) {
-        if (threadIdx.x == 0) s_task = atomicAdd(&ctl->head, 1);
-        __syncthreads();
-        const int task = s_task;
-        __syncthreads();
-        if (task >= total) break;
+    int task = int(blockIdx.x);
+    for (int turn = 0; task < total; turn ^= 1) {
+        if (threadIdx.x == 0) s_next[turn] = int(gridDim.x) + atomicAdd(&ctl->head, 1);
         int b = NB - 1;
         while (b > 0 && task >= s_first[b] + s_tasks[b]) --b;
         const int local = task - s_first[b];
@@ -229,35 +328,33 @@ __global__ void __launch_bounds__(CTA, MINB) k_sort_ragged(const typename E::Mem
             constexpr int B = decltype(bc)::value;
             constexpr int L = B + kRaggedLmin;
             if (b == B) {
-                if (fam_b)
-                    ragged_task<E, typename FamilyShape<LKB, L, CTA>::type, CTA, SB>(in, out, off, ids, s_base[B],
-                                                                                      s_count[B], local, smem_raw);
+                const int* list = ids + s_base[B];
+                if (ragged_kind<E, EW>(L) == kBlocked && fam_b)
+                    ragged_task<E, EW, L, LKB, CTA>(in, out, off, list, s_count[B], local, smem_raw);
                 else
-                    ragged_task<E, typename FamilyShape<LKA, L, CTA>::type, CTA, SB>(in, out, off, ids, s_base[B],
-                                                                                      s_count[B], local, smem_raw);
+                    ragged_task<E, EW, L, LKA, CTA>(in, out, off, list, s_count[B], local, smem_raw);
             }
         });
+        __syncthreads();
+        task = s_next[turn];
     }
 }
 
-// Shared memory of k_sort_ragged: the largest per-CTA buffer (double, or
-// single when SB) over the buckets that use it.
-template <class E, int CTA, int NB, int LKA, int LKB, bool SB>
+// Shared memory of k_sort_ragged: the largest CTA's worth of a bucket's teams.
+template <class E, class EW, int CTA, int NB, int L = kRaggedLmin>
 constexpr size_t ragged_smem() {
-    size_t best = 0;
-    for (int b = 0; b < NB; ++b) {
-        const int L = b + kRaggedLmin;
-        for (int lkf : {LKA, LKB}) {
-            const int k = family_lk(L, lkf, log2_const(CTA));
-            const int rest = L - k;
-            const int lw = rest > 5 ? rest - 5 : 0;
-            if (lw > 0) {
-                const size_t bytes = (SB ? 1 : 2) * size_t(CTA) * (size_t(1) << k) * sizeof(typename E::Reg);
-                if (bytes > best) best = bytes;
-            }
-        }
+    size_t bytes = 0;
+    if constexpr (ragged_kind<E, EW>(L) == kWindows)
+        bytes = size_t(CTA >> (L - ragged_lk<EW>())) * team_bytes<EW, ragged_lk<EW>(), L>();
+    else if constexpr (ragged_kind<E, EW>(L) == kXpose)
+        bytes = size_t(CTA >> (L - ragged_lk<EW>())) * xp_region<ragged_lk<EW>(), L - ragged_lk<EW>()>() *
+                sizeof(typename E::Reg);
+    if constexpr (L < kRaggedLmin + NB - 1) {
+        const size_t rest = ragged_smem<E, EW, CTA, NB, L + 1>();
+        return rest > bytes ? rest : bytes;
+    } else {
+        return bytes;
     }
-    return best;
 }
 
 // Launches over an id list: every array of the list fits the tile; one group

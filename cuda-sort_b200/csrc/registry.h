@@ -101,7 +101,9 @@ bool tma_set_extra_tx(unsigned int bytes);  // failure-detection test hook
 
 void register_ragged_i32(std::vector<RaggedEntry>& out);
 void register_ragged_rec(std::vector<RaggedEntry>& out);
+void register_ragged_rec_stable(std::vector<RaggedEntry>& out);
 void register_ragged_u64(std::vector<RaggedEntry>& out);
+void register_ragged_u64rec(std::vector<RaggedEntry>& out);
 
 const std::vector<RaggedEntry>& ragged_registry();
 

@@ -55,6 +55,27 @@ struct Win {
         });
         return a;
     }
+    // Natural layout: thread t holds elements [rank(t) * K, rank(t) * K + K)
+    // (its bits are in the order of the bank classes), and the inverse.
+    static __device__ __forceinline__ int rank(const int t) {
+        int r = 0;
+        sfor<0, LT>([&](auto jc) {
+            constexpr int j = decltype(jc)::value;
+            constexpr int at = P::kT.win[0].thr[j] - LK;
+            r |= ((t >> j) & 1) << at;
+        });
+        return r;
+    }
+    static __device__ __forceinline__ int thread_of(const int r) {
+        int t = 0;
+        sfor<0, LT>([&](auto jc) {
+            constexpr int j = decltype(jc)::value;
+            constexpr int at = P::kT.win[0].thr[j] - LK;
+            t |= ((r >> at) & 1) << j;
+        });
+        return t;
+    }
+
     template <int L>
     static __device__ __forceinline__ void put(const R (&v)[K], const int t, R* sm) {
         constexpr WinLayout w = layout(L);
@@ -160,20 +181,21 @@ struct Win {
     // so that only the warp has to synchronise.  `first`: index of the tile's
     // element 0 in the array of n; elements at or beyond n are padding.
     // A record buffer that is only 4-byte aligned moves word by word.
-    static __device__ __forceinline__ bool wide(const void* p) {
-        return (reinterpret_cast<uintptr_t>(p) & (sizeof(typename E::Mem) == 8 ? 7u : 3u)) == 0;
-    }
-    static __device__ __forceinline__ typename E::Mem load_one(const typename E::Mem* p, const bool w) {
-        if (w) return xp_ldcs(p);
-        return load_narrow(p);
-    }
     static __device__ __forceinline__ int io_index(const int t) { return (t & 31) | ((t >> 5) << (LK + 5)); }
 
     // Load into the natural layout.  pay: the payloads by position (gathered types).
     static __device__ __forceinline__ void load(R (&v)[K], const typename E::Mem* src, const int t, const int first,
                                                 const int n, R* sm, int32_t* pay = nullptr) {
+        if (!xp_wide(src)) {  // uniform: natural loads, and the region's padding
+            const int i0 = rank(t) * K;
+            load_tile<E, K>(v, src, first + i0, n);
+            if constexpr (gathers<E>::value)
+                if (pay)
+                    for (int i = i0; i < i0 + K && first + i < n; ++i) pay[i] = src[first + i].data;
+            put<0>(v, t, sm);
+            return;
+        }
         const int i0 = io_index(t), b = base<kIo, false>(t);
-        const bool w = wide(src);
         if constexpr (E::kStable && sizeof(R) == 16) {
             // four-word registers: the loads first, as they come from memory
             // (built into registers one by one they were waited for one by
@@ -182,7 +204,7 @@ struct Win {
             sfor<0, K>([&](auto qc) {
                 constexpr int q = decltype(qc)::value;
                 const int idx = first + i0 + 32 * q;
-                if (idx < n) m[q] = load_one(src + idx, w);
+                if (idx < n) m[q] = xp_ldcs(src + idx);
             });
             sfor<0, K>([&](auto qc) {
                 constexpr int q = decltype(qc)::value;
@@ -196,7 +218,7 @@ struct Win {
                 const int i = i0 + 32 * q, idx = first + i;
                 v[q] = E::pad();
                 if (idx < n) {
-                    const typename E::Mem m = load_one(src + idx, w);
+                    const typename E::Mem m = xp_ldcs(src + idx);
                     v[q] = E::from_mem(m, idx);
                     if constexpr (gathers<E>::value)
                         if (pay) pay[i] = m.data;
@@ -211,23 +233,32 @@ struct Win {
         __syncwarp();
         get<0>(v, t, sm);
     }
+    // Whether the tile of a whole CTA, just loaded, is in order (uniform over
+    // the CTA): each thread its elements and the first one of the next rank.
+    static __device__ __forceinline__ bool in_order(const R (&v)[K], const int t, const R* sm) {
+        __syncthreads();  // every part of the region is loaded
+        const int r = rank(t);
+        bool ok = thread_in_order<E, K>(v);
+        if (r + 1 < (1 << LT)) ok &= !E::after(v[K - 1], sh_ld(&sm[base<0, false>(thread_of(r + 1))]));
+        return __syncthreads_and(ok) != 0;
+    }
     // Store from the natural layout.
     static __device__ __forceinline__ void store(const R (&v)[K], typename E::Mem* dst, const int t, const int first,
                                                  const int n, R* sm) {
         if (dead(t, n - first)) return;
+        if (!xp_wide(dst)) {
+            store_tile<E, K>(v, dst, first + rank(t) * K, n);
+            return;
+        }
         put<0>(v, t, sm);
         __syncwarp();
         const int i0 = io_index(t), b = base<kIo, false>(t);
-        const bool w = wide(dst);
         sfor<0, K>([&](auto qc) {
             constexpr int q = decltype(qc)::value;
             constexpr int off = P::reg_off(P::kT.io, q);
             const int idx = first + i0 + 32 * q;
             const R x = sh_ld(&sm[b + off]);
-            if (idx < n) {
-                if (w) xp_stcs(dst + idx, E::to_mem(x));
-                else store_narrow(dst + idx, E::to_mem(x));
-            }
+            if (idx < n) xp_stcs(dst + idx, E::to_mem(x));
         });
     }
     // The same for gathered types: every payload is fetched (from pay when
@@ -250,13 +281,13 @@ struct Win {
             m[q] = E::to_mem(x, d);
         });
         ready();
-        const bool w = wide(dst);
+        const bool w = xp_wide(dst);
         sfor<0, K>([&](auto qc) {
             constexpr int q = decltype(qc)::value;
             const int idx = first + i0 + 32 * q;
             if (idx < n) {
                 if (w) xp_stcs(dst + idx, m[q]);
-                else store_narrow(dst + idx, m[q]);
+                else dst[idx] = m[q];
             }
         });
     }

@@ -94,14 +94,11 @@ __device__ __forceinline__ void xp_stcs(RecU64* p, const RecU64& v) {
     to_u4<0>(u, v);
     __stcs(reinterpret_cast<uint4*>(p), u);
 }
-// Records in a buffer that is only 4-byte aligned.
+// Whether whole-element accesses of p are aligned (always, but for records in
+// a buffer that is only 4-byte aligned).
 template <class M>
-__device__ __forceinline__ M load_narrow(const M* p) {
-    return *p;
-}
-template <class M>
-__device__ __forceinline__ void store_narrow(M* p, const M& v) {
-    *p = v;
+__device__ __forceinline__ bool xp_wide(const M* p) {
+    return sizeof(M) != 8 || (reinterpret_cast<uintptr_t>(p) & 7u) == 0;
 }
 
 // Element types whose tie order cannot be observed (keys alone: equal keys
@@ -444,6 +441,21 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
     }
 }
 
+// Load, sort and store the arrays of one warp (array of n elements per G-lane
+// team).  Record buffers that are only 4-byte aligned move word by word.
+template <class E, int LK, int LG, int IO>
+__device__ __forceinline__ void xp_sort_array(const typename E::Mem* src, typename E::Mem* dst, const int n,
+                                              const int t, typename E::Reg* sm) {
+    constexpr int K = 1 << LK;
+    typename E::Reg v[K];
+    if (IO == kXpIoBlocked || !xp_wide(src)) load_tile<E, K>(v, src, t * K, n);
+    else if constexpr (IO == kXpIoStaged) xp_load_staged<E, LK, LG>(v, src, t, n, sm);
+    else xp_load_striped<E, LK, LG>(v, src, t, n);
+    xp_network<E, LK, LG>(v, t, sm, false);
+    if (IO == kXpIoBlocked || !xp_wide(dst)) store_tile<E, K>(v, dst, t * K, n);
+    else xp_store_striped<E, LK, LG>(v, dst, t, n, sm);
+}
+
 // The same over a list of CSR arrays (a ragged plan's length class): arrays
 // ids[0 .. count) with array a at [off[a], off[a+1]); count and the list's
 // first position read on the device when d_count is set; each warp pulls
@@ -482,13 +494,7 @@ __global__ void __launch_bounds__(32, MINB)
             start = off[a];
             na = off[a + 1] - off[a];
         }
-        R v[K];
-        if constexpr (IO == kXpIoStaged) xp_load_staged<E, LK, LG>(v, in + start, t, na, sm);
-        else if constexpr (STRIPED) xp_load_striped<E, LK, LG>(v, in + start, t, na);
-        else load_tile<E, K>(v, in + start, t * K, na);
-        xp_network<E, LK, LG>(v, t, sm, false);
-        if constexpr (IO != kXpIoBlocked) xp_store_striped<E, LK, LG>(v, out + start, t, na, sm);
-        else store_tile<E, K>(v, out + start, t * K, na);
+        xp_sort_array<E, LK, LG, IO>(in + start, out + start, na, t, sm);
         if (!d_head) first += (long long)gridDim.x * APW;
     }
 }
