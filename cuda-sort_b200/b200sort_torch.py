@@ -24,6 +24,7 @@ or int64, arrays + 1 non-decreasing entries from 0 to N, on the same device.
 There is no CPU implementation: the operators require CUDA tensors and the
 built library, and raise otherwise.
 """
+import ctypes
 import os
 import sys
 
@@ -34,6 +35,18 @@ if HERE not in sys.path:
     sys.path.insert(0, HERE)
 
 import b200sort as bs  # noqa: E402
+
+
+def _check_offsets():
+    """The library's offset check (an internal entry point)."""
+    global _check_fn
+    if _check_fn is None:
+        p, i32, i64 = ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64
+        _check_fn = bs.declare("b200s_internal_check_offsets", ctypes.c_int, [p, i32, i64, i64, i32, p, p, p])
+    return _check_fn
+
+
+_check_fn = None
 
 
 def _dtype_of(values):
@@ -68,24 +81,26 @@ def sort_ragged(values: torch.Tensor, offsets: torch.Tensor, stable: bool = Fals
     if values.shape[0] >= 2 ** 31:
         raise RuntimeError("b200sort: ragged batches address elements with int32 offsets")
     # The kernels read elements [offsets[a], offsets[a+1]): offsets outside
-    # [0, N] or decreasing would read out of bounds, so they are checked
-    # (one device reduction and a read-back).
+    # [0, N] or decreasing would read out of bounds, so they are checked (one
+    # kernel, which also narrows int64 offsets, and a read-back).
     n_el = values.shape[0]
     top = bs.ragged_max_length(dtype, bs.STABLE if stable else 0)
-    bad = (offsets[0] != 0) | (offsets[-1] != n_el)
-    if arrays > 0:
-        lengths = offsets[1:] - offsets[:-1]
-        bad = bad | (lengths < 0).any() | (lengths > top).any()
-    if bool(bad.item()):
+    wide = offsets.dtype == torch.int64
+    src = offsets.contiguous()
+    with torch.cuda.device(values.device):
+        st = torch.cuda.current_stream(values.device).cuda_stream
+        off = torch.empty_like(src, dtype=torch.int32) if wide else src
+        bad = torch.empty(1, dtype=torch.int32, device=values.device)
+        bs.check(_check_offsets()(src.data_ptr(), int(wide), arrays, n_el, top, off.data_ptr() if wide else None,
+                                  bad.data_ptr(), st))
+    if bad.item():
         raise RuntimeError("b200sort: offsets must start at 0, end at N = %d and never decrease, and no array may "
                            "be longer than %d" % (n_el, top))
-    off = offsets if offsets.dtype == torch.int32 else offsets.to(torch.int32)
     out = torch.empty_like(values)
     if arrays == 0 or values.numel() == 0:
         return out.copy_(values)
     with torch.cuda.device(values.device):
-        st = torch.cuda.current_stream(values.device).cuda_stream
-        bs.sort_partitions(dtype, values.data_ptr(), out.data_ptr(), off.contiguous().data_ptr(), arrays, 0,
+        bs.sort_partitions(dtype, values.data_ptr(), out.data_ptr(), off.data_ptr(), arrays, 0,
                            bs.STABLE if stable else 0, st)
     return out
 
