@@ -216,23 +216,23 @@ def load_tile_table(path):
 def sort_packed(dtype, d_in, d_out, n, arrays, flags=0, tile=None, stream=0):
     """Sort `arrays` packed arrays of n elements from device pointer d_in to d_out."""
     tp = ctypes.byref(tile) if tile is not None else None
-    return check(lib().b200s_sort_packed(dtype, ctypes.c_void_p(d_in), ctypes.c_void_p(d_out), n, arrays,
-                                         flags, tp, ctypes.c_void_p(stream)))
+    return check(lib().b200s_sort_packed(dtype, d_in, d_out, n, arrays,
+                                         flags, tp, stream))
 
 
 def sort_partitions(dtype, d_in, d_out, d_counters, nb_parts, d_uniform=0, flags=0, stream=0):
     """Sort every partition [counters[p], counters[p+1]) of a partitioned array
     (the leaf of the reference's large-array sort), device pointers."""
-    return check(lib().b200s_sort_partitions(dtype, flags, ctypes.c_void_p(d_in), ctypes.c_void_p(d_out),
-                                             ctypes.c_void_p(d_counters), ctypes.c_void_p(d_uniform or None),
-                                             nb_parts, ctypes.c_void_p(stream)))
+    return check(lib().b200s_sort_partitions(dtype, flags, d_in, d_out,
+                                             d_counters, d_uniform or None,
+                                             nb_parts, stream))
 
 
 def sort_packed_status(dtype, d_in, d_out, n, arrays, flags=0, tile=None, stream=0):
     """Like sort_packed but returns the raw status code instead of raising."""
     tp = ctypes.byref(tile) if tile is not None else None
-    return lib().b200s_sort_packed(dtype, ctypes.c_void_p(d_in), ctypes.c_void_p(d_out), n, arrays, flags,
-                                   tp, ctypes.c_void_p(stream))
+    return lib().b200s_sort_packed(dtype, d_in, d_out, n, arrays, flags,
+                                   tp, stream)
 
 
 class Session:
@@ -277,16 +277,16 @@ class Plan:
         check(lib().b200s_plan_create(ctypes.byref(self._h), dtype, flags, max_arrays, device))
 
     def sort(self, d_in, d_out, d_offsets, arrays, stream=0):
-        return check(lib().b200s_sort_ragged(self._h, ctypes.c_void_p(d_in), ctypes.c_void_p(d_out),
-                                             ctypes.c_void_p(d_offsets), arrays, ctypes.c_void_p(stream)))
+        return check(lib().b200s_sort_ragged(self._h, d_in, d_out,
+                                             d_offsets, arrays, stream))
 
     def sort_hinted(self, d_in, d_out, d_offsets, h_offsets_int32, stream=0):
         """sort() with the host copy of the offsets: a plan made with
         PLAN_NO_GRAPH launches only the length classes the batch holds."""
         off = np.ascontiguousarray(h_offsets_int32, dtype=np.int32)
-        return check(lib().b200s_sort_ragged_hinted(self._h, ctypes.c_void_p(d_in), ctypes.c_void_p(d_out),
-                                                    ctypes.c_void_p(d_offsets), ctypes.c_void_p(off.ctypes.data),
-                                                    len(off) - 1, ctypes.c_void_p(stream)))
+        return check(lib().b200s_sort_ragged_hinted(self._h, d_in, d_out,
+                                                    d_offsets, off.ctypes.data,
+                                                    len(off) - 1, stream))
 
     def too_long(self, stream=0):
         c = ctypes.c_int64(0)
@@ -333,13 +333,12 @@ class Server:
         self._h = ctypes.c_void_p()
         cfg = ServerConfig(device, dtype, flags, budget_bytes, max_inflight, max_batch, max_queue)
         check(lib().b200s_server_create(ctypes.byref(self._h), ctypes.byref(cfg)))
+        self._submit = lib().b200s_server_submit
 
     def submit_status(self, src, dst, n, mem=MEM_DEVICE):
         """Raw status and ticket of one submission (src/dst are integer pointers)."""
-        t = ctypes.c_uint64(0)
-        st = lib().b200s_server_submit(self._h, ctypes.c_void_p(src), ctypes.c_void_p(dst), n, mem,
-                                       ctypes.byref(t))
-        return st, t.value
+        t = ctypes.c_uint64()
+        return self._submit(self._h, src, dst, n, mem, ctypes.byref(t)), t.value
 
     def submit(self, src, dst, n, mem=MEM_DEVICE):
         st, t = self.submit_status(src, dst, n, mem)
