@@ -76,6 +76,8 @@ struct TeamBarrierSingle {
     }
 };
 
+constexpr int log2_const(int x) { return x <= 1 ? 0 : 1 + log2_const(x / 2); }
+
 constexpr int hibit(unsigned x) {
     int b = -1;
     while (x) {

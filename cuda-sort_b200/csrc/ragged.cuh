@@ -187,8 +187,6 @@ __global__ void k_bin_scatter(const int* __restrict__ off, int arrays, RaggedCtl
                               BinSpec spec);
 #endif  // B200S_DEFINE_BIN_KERNELS
 
-constexpr int log2_const(int x) { return x <= 1 ? 0 : 1 + log2_const(x / 2); }
-
 // log2 elements per thread of bucket L (= log2 W) in a shape family with
 // K = 2^LKF: K elements per thread when a whole team fits the CTA, more when
 // it would not (the team never exceeds the CTA).

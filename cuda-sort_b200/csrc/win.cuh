@@ -76,6 +76,18 @@ struct Win {
         return t;
     }
 
+    // First element of thread t in layout kMerge (register q: q << LT further).
+    static __device__ __forceinline__ int merge_index(const int t) {
+        constexpr WinLayout w = layout(kMerge);
+        int i = 0;
+        sfor<0, LT>([&](auto jc) {
+            constexpr int j = decltype(jc)::value;
+            constexpr int at = w.thr[j];
+            i |= ((t >> j) & 1) << at;
+        });
+        return i;
+    }
+
     template <int L>
     static __device__ __forceinline__ void put(const R (&v)[K], const int t, R* sm) {
         constexpr WinLayout w = layout(L);
@@ -242,7 +254,8 @@ struct Win {
         if (r + 1 < (1 << LT)) ok &= !E::after(v[K - 1], sh_ld(&sm[base<0, false>(thread_of(r + 1))]));
         return __syncthreads_and(ok) != 0;
     }
-    // Store from the natural layout.
+    // Store from the natural layout.  KEEP: a later pass reads it again.
+    template <bool KEEP = false>
     static __device__ __forceinline__ void store(const R (&v)[K], typename E::Mem* dst, const int t, const int first,
                                                  const int n, R* sm) {
         if (dead(t, n - first)) return;
@@ -258,7 +271,10 @@ struct Win {
             constexpr int off = P::reg_off(P::kT.io, q);
             const int idx = first + i0 + 32 * q;
             const R x = sh_ld(&sm[b + off]);
-            if (idx < n) xp_stcs(dst + idx, E::to_mem(x));
+            if (idx < n) {
+                if constexpr (KEEP) xp_st(dst + idx, E::to_mem(x));
+                else xp_stcs(dst + idx, E::to_mem(x));
+            }
         });
     }
     // The same for gathered types: every payload is fetched (from pay when

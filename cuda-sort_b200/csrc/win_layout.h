@@ -90,6 +90,15 @@ constexpr WinClasses win_classes(int lk, int logw, int m) {
         }
     }
     // 4-byte elements
+    if (m == 5 && lk == 4) {
+        switch (logw) {
+            case 9: return {{3, 1, 4, 2, 3, 1, 4, 2, 0}, {5, 5, 5}};
+            case 10: return {{0, 1, 2, 4, 0, 1, 2, 3, 4, 1}, {5, 5, 5}};
+            case 11: return {{4, 3, 1, 2, 4, 3, 2, 1, 0, 0, 4}, {5, 5, 5}};
+            case 12: return {{3, 1, 2, 0, 3, 1, 0, 2, 4, 0, 3, 1}, {5, 5, 5}};
+            case 13: return {{3, 1, 2, 0, 3, 1, 0, 2, 4, 4, 5, 2, 0}, {5, 5, 5}};
+        }
+    }
     if (m == 5 && lk == 5) {
         switch (logw) {
             case 10: return {{1, 4, 3, 0, 2, 1, 3, 0, 2, 4}, {5, 5, 5}};

@@ -94,6 +94,27 @@ __device__ __forceinline__ void xp_stcs(RecU64* p, const RecU64& v) {
     to_u4<0>(u, v);
     __stcs(reinterpret_cast<uint4*>(p), u);
 }
+// The same without the streaming hint, for data that a later pass reads again.
+__device__ __forceinline__ int32_t xp_ld(const int32_t* p) { return *p; }
+__device__ __forceinline__ uint64_t xp_ld(const uint64_t* p) { return *p; }
+__device__ __forceinline__ RecI32 xp_ld(const RecI32* p) {
+    const int2 v = *reinterpret_cast<const int2*>(p);
+    return RecI32{v.x, v.y};
+}
+__device__ __forceinline__ RecU64 xp_ld(const RecU64* p) {
+    RecU64 m;
+    from_u4<0>(*reinterpret_cast<const uint4*>(p), m);
+    return m;
+}
+__device__ __forceinline__ void xp_st(int32_t* p, int32_t v) { *p = v; }
+__device__ __forceinline__ void xp_st(uint64_t* p, uint64_t v) { *p = v; }
+__device__ __forceinline__ void xp_st(RecI32* p, RecI32 v) { *reinterpret_cast<int2*>(p) = make_int2(v.key, v.data); }
+__device__ __forceinline__ void xp_st(RecU64* p, const RecU64& v) {
+    uint4 u;
+    to_u4<0>(u, v);
+    *reinterpret_cast<uint4*>(p) = u;
+}
+
 // Whether whole-element accesses of p are aligned (always, but for records in
 // a buffer that is only 4-byte aligned).
 template <class M>

@@ -18,7 +18,7 @@ def walked(tmp_path_factory):
 
 
 def test_windows_run_the_reference_network_at_unique_addresses(walked):
-    assert len(walked) == 2 * (6 + 5 + 5)
+    assert len(walked) == 2 * (6 + 5 + 5 + 5)
     assert all(ok for _, _, _, ok, _, _ in walked), walked
 
 

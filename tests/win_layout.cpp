@@ -141,6 +141,7 @@ int main() {
         range<4, 4, 9, 14>(distinct);   // records, uint64 keys, stable records
         range<4, 3, 10, 14>(distinct);  // 16-byte records
         range<5, 5, 10, 14>(distinct);  // int32 keys
+        range<4, 5, 9, 13>(distinct);   // int32 keys, 16 per thread
     }
     return 0;
 }
