@@ -346,17 +346,15 @@ struct ElemRecU64 {
         hi.key = uint64_t(b1) << 32 | b0;
     }
     // For the loops of the blocked network, where a batch of a few arrays is
-    // bound by one warp's latency: the keys by the compiler's selects, the
-    // payload on the FMA pipe (14 arrays of 345: 12.3 us as with selects alone
-    // and 14.4 with cexq; 25000 of them 280 -> 266 us).
+    // bound by one warp's latency: the compiler's selects (14 arrays of 345:
+    // 9.9 us per call, 12.5 with cexq).
     static __device__ __forceinline__ void cex(Reg& lo, Reg& hi) {
-        const uint64_t a = lo.key, b = hi.key;
-        const bool sw = b < a;
-        lo.key = sw ? b : a;
-        hi.key = sw ? a : b;
-        asm("{\n\t.reg .pred q;\n\t.reg .u32 u;\n\tsetp.lt.u64 q, %4, %3;\n\t" B200S_SWAP_FMA("0", "1", "2", "u") "}"
-            : "+r"(lo.data), "+r"(hi.data)
-            : "r"(opaque_one()), "l"(a), "l"(b));
+        const Reg a = lo, b = hi;
+        const bool sw = b.key < a.key;
+        lo.key = sw ? b.key : a.key;
+        lo.data = sw ? b.data : a.data;
+        hi.key = sw ? a.key : b.key;
+        hi.data = sw ? a.data : b.data;
     }
     static __device__ __forceinline__ Reg pick(Reg own, Reg other, bool upper) {
         const bool take = upper ? (own.key < other.key) : (other.key < own.key);
