@@ -241,6 +241,21 @@ struct ElemRecI32 {
     }
 };
 
+// The same with compare and selects: fewer instructions in all and shorter
+// code, for batches that leave the SMs mostly idle, where one warp's latency
+// and its instruction fetches count and no pipe is full (W = 256 .. 2048; see
+// kLatencyWarps in instantiate.cuh).
+struct ElemRecI32L : ElemRecI32 {
+    static __device__ __forceinline__ void cex(Reg& lo, Reg& hi) {
+        const Reg a = lo, b = hi;
+        const bool sw = b.key < a.key;
+        lo.key = sw ? b.key : a.key;
+        lo.data = sw ? b.data : a.data;
+        hi.key = sw ? a.key : b.key;
+        hi.data = sw ? a.data : b.data;
+    }
+};
+
 // Stable mode for IntAndData: (key, original position) is unique, so the
 // network output equals a stable sort by key.
 struct RegRecI32S {

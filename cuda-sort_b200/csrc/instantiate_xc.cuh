@@ -10,16 +10,17 @@
 namespace b200s {
 
 // Launch form 3 of the multi-warp tile Shape<LK, 5, LW> (one array per CTA):
-// the transposed network, attached to that tile's registry entry.
-template <class E, int LK, int LW, int MINB = 1>
+// the transposed network, attached to that tile's registry entry.  LAT: the
+// element type of its latency form (kLatencyWarps), E for none.
+template <class E, int LK, int LW, int MINB = 1, class LAT = E>
 struct PackedXc {
     using S = Shape<LK, 5, LW>;
     static constexpr int CTA = S::TPA;
     static constexpr size_t SMEM = xc_smem_bytes<E, LK, S::LOGW>();
-    template <bool CHECK>
+    template <class EL, bool CHECK>
     static cudaError_t launch_form(const void* in, void* out, int n, long long arrays, cudaStream_t st) {
         static std::atomic<unsigned long long> done{0};
-        auto fn = k_sort_packed_xc<E, S, MINB, CHECK>;
+        auto fn = k_sort_packed_xc<EL, S, MINB, CHECK>;
         cudaError_t e = opt_in_smem<SMEM>(reinterpret_cast<const void*>(fn), done);
         const auto* src = static_cast<const typename E::Mem*>(in);
         auto* dst = static_cast<typename E::Mem*>(out);
@@ -31,8 +32,10 @@ struct PackedXc {
     }
     static cudaError_t launch(const void* in, void* out, int n, long long arrays, long long,
                               cudaStream_t st, unsigned opts) {
-        return (opts & kOptSortedCheck) ? launch_form<true>(in, out, n, arrays, st)
-                                        : launch_form<false>(in, out, n, arrays, st);
+        if (opts & kOptSortedCheck) return launch_form<E, true>(in, out, n, arrays, st);
+        if (!std::is_same_v<E, LAT> && (arrays << LW) <= kLatencyWarps)
+            return launch_form<LAT, false>(in, out, n, arrays, st);
+        return launch_form<E, false>(in, out, n, arrays, st);
     }
     static cudaError_t launch_list(const void* in, void* out, const int* off, const int* ids, int count,
                                    cudaStream_t st) {

@@ -213,7 +213,7 @@ constexpr size_t team_bytes() {
 }
 
 // How the persistent kernel sorts bucket L of element type E (EW: the type
-// its windowed network runs on, ElemRecI32G for stable records):
+// its windowed and transposed networks run on, ElemRecI32G for stable records):
 //   kWindows   teams of whole warps, the windowed network of win.cuh,
 //   kXpose     several arrays per warp, the one-warp transposed network,
 //   kBlocked   shuffles and registers (network.cuh), one of two families.
@@ -261,8 +261,9 @@ __device__ __forceinline__ void ragged_task(const typename E::Mem* in, typename 
         xc_sort_array<EW, S, false>(in + start, out + start, na, t, sm, TeamBarrier{1 + team, TPA});
     } else if constexpr (ragged_kind<E, EW>(L) == kXpose) {
         constexpr int LK = ragged_lk<EW>(), LG = L - LK;
-        auto* sm = reinterpret_cast<typename E::Reg*>(smem_raw) + team * xp_region<LK, LG>();
-        xp_sort_array<E, LK, LG, keys_only<E>::value ? kXpIoStriped : kXpIoStaged>(in + start, out + start, na, t, sm);
+        auto* sm = reinterpret_cast<typename EW::Reg*>(smem_raw) + team * xp_region<LK, LG>();
+        xp_sort_array<EW, LK, LG, keys_only<EW>::value ? kXpIoStriped : kXpIoStaged>(
+            in + start, out + start, na, t, sm, xp_pay<EW, LK, LG>(smem_raw, APT, team));
     } else {
         using R = typename E::Reg;
         using S = typename FamilyShape<LKF, L, CTA>::type;
@@ -345,8 +346,7 @@ constexpr size_t ragged_smem() {
     if constexpr (ragged_kind<E, EW>(L) == kWindows)
         bytes = size_t(CTA >> (L - ragged_lk<EW>())) * team_bytes<EW, ragged_lk<EW>(), L>();
     else if constexpr (ragged_kind<E, EW>(L) == kXpose)
-        bytes = size_t(CTA >> (L - ragged_lk<EW>())) * xp_region<ragged_lk<EW>(), L - ragged_lk<EW>()>() *
-                sizeof(typename E::Reg);
+        bytes = xp_smem<EW, ragged_lk<EW>(), L - ragged_lk<EW>()>(CTA >> (L - ragged_lk<EW>()));
     if constexpr (L < kRaggedLmin + NB - 1) {
         const size_t rest = ragged_smem<E, EW, CTA, NB, L + 1>();
         return rest > bytes ? rest : bytes;

@@ -1,12 +1,13 @@
 // Transposed-network kernels (launch form 3): every comparator layer in
 // registers, the tile re-laid out through shared memory between windows
 // (xpose.cuh).  Keys (int32, uint64) read their arrays with coalesced striped
-// accesses (their input order is unobservable); IntAndData records load
-// coalesced through the shared region, keeping their order (the reference's
-// tie order depends on it).  Both store coalesced through the shared region.
+// accesses (their input order is unobservable), and so do stable records (each
+// word carries its position); IntAndData records in the reference's tie order
+// load coalesced through the shared region, keeping their order.  Both store coalesced through the shared region.
 #include <algorithm>
 #include <atomic>
 
+#include "instantiate.cuh"
 #include "xpose.cuh"
 #include "xpose_registry.h"
 
@@ -18,12 +19,16 @@ namespace {
 // bounds the registers: 28 warps per SM for int32 keys (48 registers: a
 // 4096-array batch in one wave on 148 SMs); records and 64-bit keys hold twice
 // the data per element (16 warps per SM at 32 per lane, 24 at 16).
-template <class E, int LK, int LG, int IO, int MINB_ = 28>
+// LAT: the element type of the tile's latency form (kLatencyWarps), E for none.
+template <class E, int LK, int LG, int IO, int MINB_ = 28, class LAT = E>
 struct Xpose {
     static constexpr int WPC = 1, MINB = MINB_;
     static constexpr int APW = 32 >> LG;
-    static constexpr size_t SMEM = size_t(WPC) * APW * xp_region<LK, LG>() * sizeof(typename E::Reg);
-    static constexpr auto kernel() { return k_sort_xpose<E, LK, LG, WPC, MINB, IO>; }
+    static constexpr size_t SMEM = xp_smem<E, LK, LG>(WPC * APW);
+    template <class EL = E>
+    static constexpr auto kernel() {
+        return k_sort_xpose<EL, LK, LG, WPC, MINB, IO>;
+    }
 
     // Programmatic dependent launch: the grid may be scheduled while the
     // stream's previous kernel drains; the kernel waits for that kernel's
@@ -31,18 +36,11 @@ struct Xpose {
     static cudaError_t launch(const void* in, void* out, int n, long long arrays, cudaStream_t st, unsigned opts) {
         const long long per_cta = (long long)WPC * APW;
         const long long grid = std::min<long long>((arrays + per_cta - 1) / per_cta, 0x7fffffffLL);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(unsigned(grid));
-        cfg.blockDim = dim3(WPC * 32);
-        cfg.dynamicSmemBytes = SMEM;
-        cfg.stream = st;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr.val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kernel(), static_cast<const typename E::Mem*>(in),
-                                  static_cast<typename E::Mem*>(out), n, arrays, opts);
+        const auto* src = static_cast<const typename E::Mem*>(in);
+        auto* dst = static_cast<typename E::Mem*>(out);
+        if (!std::is_same_v<E, LAT> && grid * WPC <= kLatencyWarps && !(opts & kOptSortedCheck))
+            return launch_pdl(kernel<LAT>(), unsigned(grid), WPC * 32, SMEM, st, src, dst, n, arrays, opts);
+        return launch_pdl(kernel(), unsigned(grid), WPC * 32, SMEM, st, src, dst, n, arrays, opts);
     }
     static cudaError_t attrs(cudaFuncAttributes* a) {
         return cudaFuncGetAttributes(a, reinterpret_cast<const void*>(kernel()));
@@ -98,13 +96,13 @@ const std::vector<XposeEntry>& xpose_registry() {
         constexpr int REC = 1;                                     // B200S_I32_I32, reference tie order
         v.push_back(Xpose<ElemRecI32, 5, 5, kXpIoStaged, 16>::entry(REC));  // W = 1024
         v.push_back(Xpose<ElemRecI32, 5, 4, kXpIoStaged, 16>::entry(REC));  // W = 512
-        v.push_back(Xpose<ElemRecI32, 4, 4, kXpIoStaged, 24>::entry(REC));  // W = 256
+        v.push_back(Xpose<ElemRecI32, 4, 4, kXpIoStaged, 24, ElemRecI32L>::entry(REC));  // W = 256
         v.push_back(Xpose<ElemRecI32, 4, 3, kXpIoStaged, 24>::entry(REC));  // W = 128
         v.push_back(Xpose<ElemRecI32, 4, 2, kXpIoStaged, 24>::entry(REC));  // W = 64
-        // stable records: (key, data, position) registers, 16 per lane
-        v.push_back(Xpose<ElemRecI32S, 4, 4, kXpIoStaged, 20>::entry(REC));  // W = 256
-        v.push_back(Xpose<ElemRecI32S, 4, 3, kXpIoStaged, 20>::entry(REC));  // W = 128
-        v.push_back(Xpose<ElemRecI32S, 4, 2, kXpIoStaged, 20>::entry(REC));  // W = 64
+        // stable records: 64-bit (key, position) words, the payloads aside
+        v.push_back(Xpose<ElemRecI32G, 4, 4, kXpIoStriped, 24>::entry(REC));  // W = 256
+        v.push_back(Xpose<ElemRecI32G, 4, 3, kXpIoStriped, 24>::entry(REC));  // W = 128
+        v.push_back(Xpose<ElemRecI32G, 4, 2, kXpIoStriped, 24>::entry(REC));  // W = 64
         constexpr int U64 = 2;                                     // B200S_U64
         v.push_back(Xpose<ElemU64, 5, 5, kXpIoStriped, 16>::entry(U64));    // W = 1024
         v.push_back(Xpose<ElemU64, 5, 4, kXpIoStriped, 16>::entry(U64));    // W = 512

@@ -316,11 +316,25 @@ constexpr int xp_region() {
 // 4-byte keys and G = 32) and calls them its natural-layout registers 0 .. K-1:
 // a relabelling of the input, not a data movement.  Elements at or beyond n
 // are padding.
+// Gathered types (their words carry the true position) leave the payloads in
+// pay[0 .. n).
 template <class E, int LK, int LG>
 __device__ __forceinline__ void xp_load_striped(typename E::Reg (&v)[1 << LK], const typename E::Mem* src,
-                                                const int t, const int n) {
+                                                const int t, const int n, int32_t* pay = nullptr) {
     constexpr int K = 1 << LK, G = 1 << LG;
-    if (n == K * G) {
+    if constexpr (gathers<E>::value) {
+#pragma unroll
+        for (int q = 0; q < K; ++q) {
+            const int idx = q * G + t;
+            v[q] = E::pad();
+            if (idx < n) {
+                const typename E::Mem m = xp_ldcs(src + idx);
+                v[q] = E::from_mem(m, idx);
+                pay[idx] = m.data;
+            }
+        }
+        __syncwarp();
+    } else if (n == K * G) {
 #pragma unroll
         for (int q = 0; q < K; ++q) v[q] = E::from_mem(xp_ldcs(src + q * G + t), q * G + t);
     } else {
@@ -367,7 +381,8 @@ __device__ __forceinline__ void xp_load_staged(typename E::Reg (&v)[1 << LK], co
 // warp's other arrays sit G banks further on).
 template <class E, int LK, int LG>
 __device__ __forceinline__ void xp_store_striped(typename E::Reg (&v)[1 << LK], typename E::Mem* dst,
-                                                 const int t, const int n, typename E::Reg* sm) {
+                                                 const int t, const int n, typename E::Reg* sm,
+                                                 const int32_t* pay = nullptr) {
     constexpr int K = 1 << LK, G = 1 << LG;
     const int bn = xp_addr<LK>(t << LK);
     sfor<0, K>([&](auto qc) {
@@ -375,7 +390,19 @@ __device__ __forceinline__ void xp_store_striped(typename E::Reg (&v)[1 << LK], 
         sm[bn + xp_addr<LK>(q)] = v[q];
     });
     __syncwarp();
-    if (n == K * G) {
+    if constexpr (gathers<E>::value) {
+        const bool wide = xp_wide(dst);
+#pragma unroll
+        for (int q = 0; q < K; ++q) {
+            const int idx = q * G + t;
+            const typename E::Reg x = sm[xp_addr<LK>(idx)];
+            if (idx < n) {
+                const typename E::Mem m = E::to_mem(x, pay[E::position(x)]);
+                if (wide) xp_stcs(dst + idx, m);
+                else dst[idx] = m;
+            }
+        }
+    } else if (n == K * G) {
 #pragma unroll
         for (int q = 0; q < K; ++q) xp_stcs(dst + q * G + t, E::to_mem(sm[xp_addr<LK>(q * G + t)]));
     } else {
@@ -387,6 +414,34 @@ __device__ __forceinline__ void xp_store_striped(typename E::Reg (&v)[1 << LK], 
         }
     }
     __syncwarp();
+}
+
+// Load in natural order straight from memory (the sortedness check, record
+// buffers that are only 4-byte aligned); payloads of gathered types to pay.
+template <class E, int LK>
+__device__ __forceinline__ void xp_load_natural(typename E::Reg (&v)[1 << LK], const typename E::Mem* src,
+                                                const int t, const int n, int32_t* pay) {
+    constexpr int K = 1 << LK;
+    load_tile<E, K>(v, src, t * K, n);
+    if constexpr (gathers<E>::value) {
+        for (int i = t * K; i < t * K + K && i < n; ++i) pay[i] = src[i].data;
+        __syncwarp();
+    }
+}
+
+// Shared-memory bytes of `teams` arrays: their regions, then the payloads of
+// gathered types.
+template <class E, int LK, int LG>
+constexpr size_t xp_smem(int teams) {
+    return size_t(teams) * (xp_region<LK, LG>() * sizeof(typename E::Reg) +
+                            (gathers<E>::value ? size_t(4) << (LK + LG) : 0));
+}
+template <class E, int LK, int LG>
+__device__ __forceinline__ int32_t* xp_pay(void* smem, const int teams, const int team) {
+    if constexpr (gathers<E>::value)
+        return reinterpret_cast<int32_t*>(static_cast<typename E::Reg*>(smem) + teams * xp_region<LK, LG>()) +
+               (team << (LK + LG));
+    else return nullptr;
 }
 
 // Packed batch (array a at [a*n, a*n + n)): each warp sorts 32/G arrays at a
@@ -407,11 +462,12 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
     using R = typename E::Reg;
     constexpr int K = 1 << LK, G = 1 << LG, APW = 32 / G;
     static_assert(LG <= 5 && LG <= LK && LG >= 1, "one warp or less per array, at most two windows");
-    static_assert(!STRIPED || !E::kStable, "striped access relabels the input: keys only");
+    static_assert(!STRIPED || !E::kStable || gathers<E>::value, "striped access relabels the input: keys only");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = int(threadIdx.x) >> 5, lane = int(threadIdx.x) & 31;
     const int slot = lane >> LG, t = lane & (G - 1);
     R* sm = reinterpret_cast<R*>(smem_raw) + (warp * APW + slot) * xp_region<LK, LG>();
+    int32_t* pay = xp_pay<E, LK, LG>(smem_raw, WPC * APW, warp * APW + slot);
     const long long stride = (long long)gridDim.x * WPC * APW;
     // Launched with programmatic stream serialization: wait until the
     // preceding kernel of the stream has completed and its writes are
@@ -429,8 +485,8 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
         if constexpr (IO == kXpIoStaged) {
             xp_load_staged<E, LK, LG>(x, src, t, na, sm);
         } else {
-            if (STRIPED && !check) xp_load_striped<E, LK, LG>(x, src, t, na);
-            else load_tile<E, K>(x, src, t * K, na);
+            if (STRIPED && !check) xp_load_striped<E, LK, LG>(x, src, t, na, pay);
+            else xp_load_natural<E, LK>(x, src, t, na, pay);
         }
     };
     auto finish = [&](R (&x)[K], long long a) {
@@ -440,7 +496,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
         if (skip && in == out) return;  // in order and in place: nothing to write
         const int na = a < arrays ? n : 0;
         typename E::Mem* dst = out + (a < arrays ? a : 0) * (long long)n;
-        if constexpr (IO != kXpIoBlocked) xp_store_striped<E, LK, LG>(x, dst, t, na, sm);
+        if constexpr (IO != kXpIoBlocked) xp_store_striped<E, LK, LG>(x, dst, t, na, sm, pay);
         else store_tile<E, K>(x, dst, t * K, na);
     };
     R v[K];
@@ -466,15 +522,20 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
 // team).  Record buffers that are only 4-byte aligned move word by word.
 template <class E, int LK, int LG, int IO>
 __device__ __forceinline__ void xp_sort_array(const typename E::Mem* src, typename E::Mem* dst, const int n,
-                                              const int t, typename E::Reg* sm) {
+                                              const int t, typename E::Reg* sm, int32_t* pay = nullptr) {
     constexpr int K = 1 << LK;
     typename E::Reg v[K];
-    if (IO == kXpIoBlocked || !xp_wide(src)) load_tile<E, K>(v, src, t * K, n);
+    if (IO == kXpIoBlocked || !xp_wide(src)) xp_load_natural<E, LK>(v, src, t, n, pay);
     else if constexpr (IO == kXpIoStaged) xp_load_staged<E, LK, LG>(v, src, t, n, sm);
-    else xp_load_striped<E, LK, LG>(v, src, t, n);
+    else xp_load_striped<E, LK, LG>(v, src, t, n, pay);
     xp_network<E, LK, LG>(v, t, sm, false);
-    if (IO == kXpIoBlocked || !xp_wide(dst)) store_tile<E, K>(v, dst, t * K, n);
-    else xp_store_striped<E, LK, LG>(v, dst, t, n, sm);
+    if constexpr (gathers<E>::value) {
+        xp_store_striped<E, LK, LG>(v, dst, t, n, sm, pay);
+    } else if (IO == kXpIoBlocked || !xp_wide(dst)) {
+        store_tile<E, K>(v, dst, t * K, n);
+    } else {
+        xp_store_striped<E, LK, LG>(v, dst, t, n, sm);
+    }
 }
 
 // The same over a list of CSR arrays (a ragged plan's length class): arrays
@@ -490,11 +551,12 @@ __global__ void __launch_bounds__(32, MINB)
     using R = typename E::Reg;
     constexpr int K = 1 << LK, G = 1 << LG, APW = 32 / G;
     static_assert(LG <= 5 && LG <= LK && LG >= 1, "one warp or less per array, at most two windows");
-    static_assert(!STRIPED || !E::kStable, "striped access relabels the input: keys only");
+    static_assert(!STRIPED || !E::kStable || gathers<E>::value, "striped access relabels the input: keys only");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = int(threadIdx.x) & 31;
     const int slot = lane >> LG, t = lane & (G - 1);
     R* sm = reinterpret_cast<R*>(smem_raw) + slot * xp_region<LK, LG>();
+    int32_t* pay = xp_pay<E, LK, LG>(smem_raw, APW, slot);
     if (d_count) {
         count = *d_count;
         ids += *d_base;
@@ -515,7 +577,7 @@ __global__ void __launch_bounds__(32, MINB)
             start = off[a];
             na = off[a + 1] - off[a];
         }
-        xp_sort_array<E, LK, LG, IO>(in + start, out + start, na, t, sm);
+        xp_sort_array<E, LK, LG, IO>(in + start, out + start, na, t, sm, pay);
         if (!d_head) first += (long long)gridDim.x * APW;
     }
 }
