@@ -20,8 +20,7 @@ lengths log-uniform in [1, 8192], records; the plan's launch sequence
 replayed from its CUDA graph, with one launch per length class and the
 plain per-length launches timed beside it), cluster_256x65536 /
 cluster_u64_256x65536 (256 arrays of 65536 records with int32 / uint64
-keys, one thread-block cluster per array: 4 CTAs of 1024 threads / 8 CTAs
-of 512),
+keys, longer than one CTA holds: sorted in passes over global memory),
 serving (a stream of sort requests of 16 .. 65536 records into the
 continuous-batching server under a 16 GB device budget: peak sustained keys/s
 in closed loop, then Poisson arrival rates with p50/p99/p99.9 latency, each
@@ -482,7 +481,8 @@ def _batched_inplace_us(ctx, launch, sets, pristine, flush, passes):
     return statistics.median(times)
 
 
-def gpu_baselines(ctx, wl, data, host, ours_tile):
+def gpu_baselines(ctx, wl, data, host, ours_tile, default_route=False):
+    """default_route: ours runs without a tile request (the sort in passes)."""
     torch = ctx.torch
     dtype, n, arrays, flags = wl["dtype"], wl["n"], wl["arrays"], wl["flags"]
     npd = bs.NP_DTYPES[dtype]
@@ -515,7 +515,9 @@ def gpu_baselines(ctx, wl, data, host, ours_tile):
         out[name] = {"us": us, "config": best[0], "verified": us is not None and check()}
 
     st = ctx.sh
-    family("ours", [(repr(ours_tile), lambda p: bs.sort_packed_status(dtype, p, p, n, arrays, flags, ours_tile, st))])
+    ours = None if default_route else ours_tile
+    family("ours", [("in passes" if default_route else repr(ours_tile),
+                     lambda p: bs.sort_packed_status(dtype, p, p, n, arrays, flags, ours, st))])
     plain = ours_tile.with_form(0)
     family("plain", [(repr(plain), lambda p: bs.sort_packed_status(dtype, p, p, n, arrays, flags, plain, st))])
     plain_flags = flags & ~bs.SORTED_CHECK
@@ -660,14 +662,22 @@ def run_gpu(args, wl):
         cluster = info.arrays_per_cta == 0
         if form == 3 and not info.xpose_form:
             form = 0
-        if form == 3:
+        # arrays beyond one CTA without a tile request are sorted in passes (one
+        # launch for the slices, two per stage above them); the tile's CTA
+        # bits count the stages only when the tile was asked for
+        passes = cluster and tile is None and not (flags & bs.STABLE)
+        slice_bits = 13 if dtype == bs.U64_I32 else 14
+        stages = max(0, int(n - 1).bit_length() - slice_bits) if passes else 0
+        if passes:
+            kernel = "k_sort_slices, k_merge_far, k_merge_near"
+        elif form == 3:
             kernel = "k_sort_cluster_xc" if cluster else "k_sort_packed_xc" if eff.log2_warps > 0 else "k_sort_xpose"
         else:
             kernel = "k_sort_cluster" if cluster else {0: "k_sort_packed", 1: "k_sort_packed_pf",
                                                        2: "k_sort_packed_tma"}[form]
-        launches = args.steps
+        launches = args.steps * (1 + 2 * stages)
         if ctx.world == 1 and not args.no_baselines:
-            extra["baselines"] = gpu_baselines(ctx, wl, data, host, eff)
+            extra["baselines"] = gpu_baselines(ctx, wl, data, host, eff, passes)
     else:
         arrays = wl["arrays"]
         d_in = host.to(ctx.dev)
@@ -682,7 +692,9 @@ def run_gpu(args, wl):
         got = d_out.cpu().numpy().view(bs.NP_DTYPES[dtype])
         verified = verify_ragged(dtype, data, off, got) and plan.too_long(ctx.sh) == 0
         kernel = "k_sort_ragged"
-        launches = 3 * args.steps   # bin count, bin scatter, sort (one graph per step)
+        # bin count, bin scatter, the persistent sort and a launch per cluster
+        # class (lengths beyond its classes), in one graph per step
+        launches = (3 + (bs.ragged_max_length(dtype, flags).bit_length() - 14)) * args.steps
     if wl["kind"] == "ragged" and not args.no_plain:
         # the plain per-length launches on the same input
         plain_launches = plan.prepare_plain(off.astype(np.int32))
@@ -722,10 +734,13 @@ def run_gpu(args, wl):
     t_hbm = algo_bytes / (hbm * 1e9)
     if wl["kind"] == "packed":
         w = 1 << (eff.log2_items + eff.log2_lanes + eff.log2_warps + eff.log2_ctas)
-        roofline["alu"] = alu_roofline(dtype, eff, wl["arrays"] * w, ms_step * 1e-3, clocks.get("sm_mhz"), form)
+        alu_tile = bs.Tile(eff.log2_items, eff.log2_lanes, eff.log2_warps + eff.log2_ctas, 0, form, 0) \
+            if passes else eff
+        roofline["alu"] = alu_roofline(dtype, alu_tile, wl["arrays"] * w, ms_step * 1e-3, clocks.get("sm_mhz"), form)
         wmin = 1 << max(5, int(wl["n"] - 1).bit_length())
         roofline["onchip"] = onchip_roofline(np.full(wl["arrays"], wmin), bs.ELEM_BYTES[dtype], ms_step * 1e-3,
-                                             t_hbm, ctx.local, lc=eff.log2_ctas, arrays=wl["arrays"])
+                                             t_hbm, ctx.local, lc=0 if passes else eff.log2_ctas,
+                                             arrays=wl["arrays"])
     else:
         lens = np.diff(off).astype(np.int64)
         lens = lens[lens > 0]

@@ -1,4 +1,4 @@
-// Launch form 3 of the IntAndData record cluster tiles: the transposed
+// Launch form 3 of the IntAndData record cluster tiles: the windowed
 // network of cta_xpose.cuh (1024-thread CTAs of 16384 records, and the
 // 512-thread latency alternatives).
 #include "instantiate_xc.cuh"

@@ -1,5 +1,5 @@
 // Launch form 3 of the multi-warp and cluster tiles of int32 and uint64 keys:
-// the transposed network of cta_xpose.cuh (one array per CTA or cluster).
+// the windowed network of cta_xpose.cuh (one array per CTA or cluster).
 // MINB keeps every tile at 64 registers per thread or fewer.
 #include "instantiate_xc.cuh"
 

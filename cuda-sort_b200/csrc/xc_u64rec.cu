@@ -1,5 +1,5 @@
 // Launch form 3 of the {uint64 key, int32 payload} record tiles: the
-// transposed network of cta_xpose.cuh for the multi-warp tiles (W up to
+// windowed network of cta_xpose.cuh for the multi-warp tiles (W up to
 // 4096) and the 8192-record-per-CTA cluster tiles (W up to 65536).
 #include "instantiate_xc.cuh"
 

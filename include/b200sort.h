@@ -155,8 +155,12 @@ b200s_status b200s_load_tile_table(const char* path, int32_t* applied);
 
 /* Sort `arrays` independent arrays of n elements each, packed back to back
  * (array a at element offset a*n), from d_in into d_out (device pointers; may
- * be equal).  tile == NULL uses the default tile for n.  The single-CTA
- * launches allow programmatic stream serialization: their CTAs may be
+ * be equal).  tile == NULL uses the default tile for n, or, for arrays longer
+ * than one CTA holds and for small batches of arrays beyond 4096 elements, a
+ * sort in passes: one launch for slices of the arrays and two per later stage
+ * of the network, in place in d_out, with the same output (not for stable
+ * records, nor for record buffers that are only 4-byte aligned).  The single-CTA
+ * launches and the passes allow programmatic stream serialization: their CTAs may be
  * scheduled while the stream's previous kernel drains, and each waits for
  * that kernel's completion (griddepcontrol.wait) before touching memory, so
  * stream order is kept for any producer. */
@@ -168,8 +172,10 @@ b200s_status b200s_sort_packed(b200s_dtype dtype, const void* d_in, void* d_out,
  * Array a occupies elements [offsets[a], offsets[a+1]) of the flat buffer
  * (int32 offsets, arrays + 1 entries, non-decreasing).  A plan owns the
  * scratch of the bucketed launch (a control block and 2 * max_arrays ids)
- * and, unless B200S_PLAN_NO_GRAPH is set, a CUDA graph of the launch
- * sequence, re-captured when the buffers or the array count change.  Replaces
+ * and, unless B200S_PLAN_NO_GRAPH is set, a CUDA graph of the launch sequence:
+ * a call with the previous call's buffers and array count captures and replays
+ * it; a call with others, or on a stream that is being captured, launches the
+ * sequence directly.  Calls of one plan on different streams are ordered.  Replaces
  * the reference's partition sort over CSR partitions
  * (SortPartitionsAdaptive_outofplace, cusort.hpp:2309-2352). */
 typedef struct b200s_plan b200s_plan;
@@ -181,8 +187,7 @@ int32_t b200s_ragged_max_length(b200s_dtype dtype, uint32_t flags);
 /* The plan's launch sequence: binning, then the persistent length-bucketed
  * kernel on `stream`, with the length classes that the tile table gives a
  * launch of their own and the cluster classes above the persistent kernel's
- * range on side streams, joined before return (graph-replayed unless
- * B200S_PLAN_NO_GRAPH). */
+ * range on side streams, joined before return. */
 b200s_status b200s_sort_ragged(b200s_plan* plan, const void* d_in, void* d_out, const int32_t* d_offsets,
                                int64_t arrays, void* stream);
 /* b200s_sort_ragged for a caller that also holds the offsets on the host
@@ -190,7 +195,8 @@ b200s_status b200s_sort_ragged(b200s_plan* plan, const void* d_in, void* d_out, 
  * A B200S_PLAN_NO_GRAPH plan then issues only the launches of the length
  * classes the batch holds: a launch of its own or a cluster class that no
  * array falls in is skipped, and so is the persistent kernel when every
- * array is in such a class.  Results equal b200s_sort_ragged's.  A graph plan
+ * array is in such a class; a cluster class of a few arrays runs with more
+ * CTAs per array.  Results equal b200s_sort_ragged's.  A graph plan
  * (or h_offsets == NULL) runs b200s_sort_ragged. */
 b200s_status b200s_sort_ragged_hinted(b200s_plan* plan, const void* d_in, void* d_out, const int32_t* d_offsets,
                                       const int32_t* h_offsets, int64_t arrays, void* stream);
@@ -223,7 +229,7 @@ int32_t b200s_plan_plain_launches(const b200s_plan* plan);
  * 48 KB rule to a separate merge sort); longer ones are not written to d_out,
  * and the caller sorts them as the reference's merge path does.
  * Backed by a ragged plan cached per device, element type and stream (one
- * allocation the first time, re-captured graph when the buffers change);
+ * allocation the first time);
  * b200s_release_partition_plans frees the cached plans. */
 b200s_status b200s_sort_partitions(b200s_dtype dtype, uint32_t flags, const void* d_in, void* d_out,
                                    const int32_t* d_counters, const int32_t* d_uniform, int32_t nb_parts,
