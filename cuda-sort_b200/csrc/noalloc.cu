@@ -136,7 +136,7 @@ extern "C" b200s_status b200s_sort_ragged_noalloc(b200s_dtype dtype, uint32_t fl
     dedicated_entries(dtype, stable, rk->nb, &dedicated, dedicated_idx, dedicated_xc);
     if (dedicated != (1u << rk->nb) - 1u) {
         e = rk->launch(d_in, d_out, d_offsets, s->ids, &s->ctl, ragged_family_mask(dtype, stable), dedicated,
-                       sms * per_sm, cs);
+                       std::max(1, std::min(sms * per_sm, n)), cs);
         if (e != cudaSuccess) return cuda_error(e, "ragged sort launch");
     }
     for (int b = rk->nb - 1; b >= 0; --b) {

@@ -277,7 +277,9 @@ b200s_status record_sequence(b200s_plan* p, const void* in, void* out, const int
     }
     const uint32_t all = (1u << p->spec.nb) - 1u;
     if (present & all & ~p->dedicated_mask) {
-        e = p->rk->launch(in, out, off, p->ids, p->ctl, p->family_mask, p->dedicated_mask, p->grid, st);
+        // a task holds at least one array: a small batch needs no full grid
+        e = p->rk->launch(in, out, off, p->ids, p->ctl, p->family_mask, p->dedicated_mask,
+                          std::max(1, std::min(p->grid, arrays)), st);
         if (e != cudaSuccess) return cuda_error(e, "ragged sort launch");
     }
     for (int s = 0; s < used; ++s) {
