@@ -63,19 +63,6 @@ struct TeamBarrier {
         asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
     }
 };
-// The same with one shared-memory buffer per team (see single_buffer below).
-struct TeamBarrierSingle {
-    static constexpr bool kSingleBuffer = true;
-    int id;
-    int threads;
-    __device__ __forceinline__ void operator()() const {
-        asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-    }
-    __device__ __forceinline__ void unaligned() const {
-        asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-    }
-};
-
 constexpr int log2_const(int x) { return x <= 1 ? 0 : 1 + log2_const(x / 2); }
 
 constexpr int hibit(unsigned x) {

@@ -208,40 +208,24 @@ struct Win {
             return;
         }
         const int i0 = io_index(t), b = base<kIo, false>(t);
-        if constexpr (E::kStable && sizeof(R) == 16) {
-            // four-word registers: the loads first, as they come from memory
-            // (built into registers one by one they were waited for one by
-            // one: 127 -> 100 us at W = 1024)
-            typename E::Mem m[K];
-            sfor<0, K>([&](auto qc) {
-                constexpr int q = decltype(qc)::value;
-                const int idx = first + i0 + 32 * q;
-                if (idx < n) m[q] = xp_ldcs(src + idx);
-            });
-            sfor<0, K>([&](auto qc) {
-                constexpr int q = decltype(qc)::value;
-                constexpr int off = P::reg_off(P::kT.io, q);
-                const int idx = first + i0 + 32 * q;
-                sh_st(&sm[b + off], idx < n ? E::from_mem(m[q], idx) : E::pad());
-            });
-        } else {
-            sfor<0, K>([&](auto qc) {
-                constexpr int q = decltype(qc)::value;
-                const int i = i0 + 32 * q, idx = first + i;
-                v[q] = E::pad();
-                if (idx < n) {
-                    const typename E::Mem m = xp_ldcs(src + idx);
-                    v[q] = E::from_mem(m, idx);
-                    if constexpr (gathers<E>::value)
-                        if (pay) pay[i] = m.data;
-                }
-            });
-            sfor<0, K>([&](auto qc) {
-                constexpr int q = decltype(qc)::value;
-                constexpr int off = P::reg_off(P::kT.io, q);
-                sh_st(&sm[b + off], v[q]);
-            });
-        }
+        // The loads first, as they come from memory, and the payloads stored
+        // without a branch: a store inside the bounds test kept the loads of
+        // gathered types apart (4 M stable records, W = 1024 / 2048 / 4096:
+        // 68.6 / 76.7 / 83.3 -> 57.6 / 67.0 / 76.7 us).
+        typename E::Mem m[K];
+        sfor<0, K>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            const int idx = first + i0 + 32 * q;
+            if (idx < n) m[q] = xp_ldcs(src + idx);
+        });
+        sfor<0, K>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            constexpr int off = P::reg_off(P::kT.io, q);
+            const int i = i0 + 32 * q, idx = first + i;
+            if constexpr (gathers<E>::value)
+                if (pay) pay[i] = m[q].data;
+            sh_st(&sm[b + off], idx < n ? E::from_mem(m[q], idx) : E::pad());
+        });
         __syncwarp();
         get<0>(v, t, sm);
     }

@@ -266,22 +266,8 @@ struct WinPlan {
             if ((q >> r) & 1) a += kT.weight[w.reg[r]];
         return a;
     }
-    // Index part of register q in a layout.
-    static constexpr int reg_index(const WinLayout& w, int q) {
-        int i = 0;
-        for (int r = 0; r < LK; ++r)
-            if ((q >> r) & 1) i |= 1 << w.reg[r];
-        return i;
-    }
     // Whether register q of window w is stored with complemented thread bits.
     static constexpr bool mirrored(const WinLayout& w, int q) { return w.refl >= 0 && ((q >> w.refl) & 1); }
-    // Element index held by register 0 of a thread whose bits are t (not mirrored).
-    static constexpr int thread_index(const WinLayout& w, int t) {
-        int i = 0;
-        for (int j = 0; j < LT; ++j)
-            if ((t >> j) & 1) i |= 1 << w.thr[j];
-        return i;
-    }
     // Whether every warp holds the same part of the tile in both layouts.
     static constexpr bool same_warps(const WinLayout& a, const WinLayout& b) {
         for (int j = LG; j < LT; ++j)

@@ -323,15 +323,15 @@ __device__ __forceinline__ void xp_load_striped(typename E::Reg (&v)[1 << LK], c
                                                 const int t, const int n, int32_t* pay = nullptr) {
     constexpr int K = 1 << LK, G = 1 << LG;
     if constexpr (gathers<E>::value) {
+        typename E::Mem m[K];  // the loads first, the payloads without a branch (see Win::load)
+#pragma unroll
+        for (int q = 0; q < K; ++q)
+            if (q * G + t < n) m[q] = xp_ldcs(src + q * G + t);
 #pragma unroll
         for (int q = 0; q < K; ++q) {
             const int idx = q * G + t;
-            v[q] = E::pad();
-            if (idx < n) {
-                const typename E::Mem m = xp_ldcs(src + idx);
-                v[q] = E::from_mem(m, idx);
-                pay[idx] = m.data;
-            }
+            pay[idx] = m[q].data;
+            v[q] = idx < n ? E::from_mem(m[q], idx) : E::pad();
         }
         __syncwarp();
     } else if (n == K * G) {
