@@ -86,8 +86,11 @@ __global__ void k_bin_count(const int* __restrict__ off, int arrays, RaggedCtl* 
 // between the two halves.  One launch of about 3 us where the reset and the
 // two kernels below take three launches in a row; from several thousand
 // arrays on one CTA's loads and list stores take longer than that.
-__global__ void __launch_bounds__(1024) k_bin_small(const int* __restrict__ off, int arrays, RaggedCtl* ctl, int* ids,
-                                                    int* oids, BinSpec spec) {
+// (Offsets and lists of a kernel launched with programmatic stream
+// serialization are not __restrict__: that would promise that they are constant
+// from the kernel's start, before griddepcontrol.wait, and allow loads above it.)
+__global__ void __launch_bounds__(1024) k_bin_small(const int* off, int arrays, RaggedCtl* ctl, int* ids, int* oids,
+                                                    BinSpec spec) {
     constexpr int kPer = kBinSmall / 1024, kClasses = kMaxBuckets + kMaxOverflow;
     __shared__ int h[kClasses + 1], base[kMaxBuckets];  // h[kClasses]: too long for every kernel
     const int t = int(threadIdx.x), lane = t & 31;
@@ -180,8 +183,7 @@ __global__ void k_bin_scatter(const int* __restrict__ off, int arrays, RaggedCtl
     }
 }
 #else
-__global__ void k_bin_small(const int* __restrict__ off, int arrays, RaggedCtl* ctl, int* ids, int* oids,
-                            BinSpec spec);
+__global__ void k_bin_small(const int* off, int arrays, RaggedCtl* ctl, int* ids, int* oids, BinSpec spec);
 __global__ void k_bin_count(const int* __restrict__ off, int arrays, RaggedCtl* ctl, BinSpec spec);
 __global__ void k_bin_scatter(const int* __restrict__ off, int arrays, RaggedCtl* ctl, int* ids, int* oids,
                               BinSpec spec);
@@ -239,8 +241,8 @@ constexpr int ragged_log_tpa(int L, int family_k, int log_cta) {
 
 template <class E, class EW, int L, int LKF, int CTA>
 __device__ __forceinline__ void ragged_task(const typename E::Mem* in, typename E::Mem* out,
-                                            const int* __restrict__ off, const int* __restrict__ ids,
-                                            const int count, const int local_task, unsigned char* smem_raw) {
+                                            const int* off, const int* ids, const int count,
+                                            const int local_task, unsigned char* smem_raw) {
     constexpr int LOGTPA = ragged_log_tpa<E, EW>(L, LKF, log2_const(CTA)), TPA = 1 << LOGTPA;
     static_assert(TPA <= CTA, "a team fits the CTA");
     constexpr int APT = CTA / TPA;
@@ -285,8 +287,7 @@ __device__ __forceinline__ void ragged_task(const typename E::Mem* in, typename 
 // from the queue, each drawn while the previous task is sorted.
 template <class E, class EW, int CTA, int NB, int LKA, int LKB, int MINB>
 __global__ void __launch_bounds__(CTA, MINB) k_sort_ragged(const typename E::Mem* in, typename E::Mem* out,
-                                                        const int* __restrict__ off,
-                                                        const int* __restrict__ ids, RaggedCtl* ctl,
+                                                        const int* off, const int* ids, RaggedCtl* ctl,
                                                         unsigned family_mask, unsigned dedicated_mask) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_first[NB], s_tasks[NB], s_base[NB], s_count[NB];
