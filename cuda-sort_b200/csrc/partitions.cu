@@ -15,10 +15,14 @@
 // graph).  Plans are cached per (device, element type, stable, stream) and
 // grown to the largest partition count seen; b200s_release_partition_plans
 // frees them.  Calls on one stream are ordered by the stream; calls on
-// different streams use different plans.
+// different streams use different plans.  A plan serves one call at a time: a
+// call holds its entry until its whole sequence is enqueued, so that the
+// launches of two host threads on one stream do not mix on one control block,
+// and no other call grows or frees the plan meanwhile.
 #include <cuda_runtime.h>
 
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <tuple>
@@ -36,14 +40,22 @@ using namespace b200s;
 namespace {
 
 struct CachedPlan {
+    std::mutex mutex;  // held from the lookup of the plan to the end of the call
     b200s_plan* plan = nullptr;
     int64_t capacity = 0;
+    void reset() {
+        if (plan) b200s_plan_destroy(plan);
+        plan = nullptr;
+        capacity = 0;
+    }
+    ~CachedPlan() { reset(); }  // released while a call was waiting for it: the last such call frees it
 };
 using PlanKey = std::tuple<int, int, int, void*>;  // device, dtype, stable, stream
-std::mutex g_plan_mutex;
-std::map<PlanKey, CachedPlan>& plan_cache() {
-    static std::map<PlanKey, CachedPlan> cache;
-    return cache;
+using PlanCache = std::map<PlanKey, std::shared_ptr<CachedPlan>>;
+std::mutex g_plan_mutex;  // the map only
+PlanCache& plan_cache() {
+    static PlanCache* cache = new PlanCache;  // never destroyed: the device may be gone at exit
+    return *cache;
 }
 
 }  // namespace
@@ -64,30 +76,35 @@ b200s_status b200s_sort_partitions(b200s_dtype dtype, uint32_t flags, const void
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return cuda_error(e, "cudaGetDevice");
     const int stable = effective_stable(dtype, flags);
-    b200s_plan* plan = nullptr;
+    std::shared_ptr<CachedPlan> c;
     {
         std::lock_guard<std::mutex> lock(g_plan_mutex);
-        CachedPlan& c = plan_cache()[PlanKey(dev, int(dtype), stable, stream)];
-        if (c.capacity < nb_parts) {
-            if (c.plan) b200s_plan_destroy(c.plan);
-            c.plan = nullptr;
-            c.capacity = 0;
-            int64_t cap = 1024;  // the reference's partition count limit (MaxNbParts)
-            while (cap < nb_parts) cap *= 2;
-            const b200s_status st = b200s_plan_create(&c.plan, dtype, stable ? B200S_STABLE : 0u, cap, dev);
-            if (st != B200S_OK) return st;
-            c.capacity = cap;
-        }
-        plan = c.plan;
+        std::shared_ptr<CachedPlan>& entry = plan_cache()[PlanKey(dev, int(dtype), stable, stream)];
+        if (!entry) entry = std::make_shared<CachedPlan>();
+        c = entry;
     }
-    return b200s_sort_ragged(plan, d_in, d_out, d_counters, nb_parts, stream);
+    std::lock_guard<std::mutex> lock(c->mutex);
+    if (c->capacity < nb_parts) {
+        c->reset();
+        int64_t cap = 1024;  // the reference's partition count limit (MaxNbParts)
+        while (cap < nb_parts) cap *= 2;
+        const b200s_status st = b200s_plan_create(&c->plan, dtype, stable ? B200S_STABLE : 0u, cap, dev);
+        if (st != B200S_OK) return st;
+        c->capacity = cap;
+    }
+    return b200s_sort_ragged(c->plan, d_in, d_out, d_counters, nb_parts, stream);
 }
 
 b200s_status b200s_release_partition_plans(void) {
-    std::lock_guard<std::mutex> lock(g_plan_mutex);
-    for (auto& kv : plan_cache())
-        if (kv.second.plan) b200s_plan_destroy(kv.second.plan);
-    plan_cache().clear();
+    PlanCache old;
+    {
+        std::lock_guard<std::mutex> lock(g_plan_mutex);
+        old.swap(plan_cache());
+    }
+    for (auto& kv : old) {
+        std::lock_guard<std::mutex> lock(kv.second->mutex);
+        kv.second->reset();
+    }
     return B200S_OK;
 }
 
