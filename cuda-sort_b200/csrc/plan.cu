@@ -206,7 +206,7 @@ struct b200s_plan {
     cudaStream_t side[kSides] = {};  // cluster and dedicated buckets run beside the persistent kernel
     cudaEvent_t fork = nullptr, join[kSides] = {};
     cudaEvent_t done = nullptr;           // end of the last call: calls on another stream wait for it
-    cudaStream_t last_stream = nullptr;
+    unsigned long long last_stream = 0;   // cudaStreamGetId of its stream
     bool used = false;
     // The buffers and array count of a call; the graph's and the last call's.
     struct Call {
@@ -290,19 +290,22 @@ b200s_status record_sequence(b200s_plan* p, const void* in, void* out, const int
 }
 
 // Calls share the plan's scratch: one on another stream than the last waits
-// for that one's end.  (Inside a stream capture the order is the caller's.)
-b200s_status begin_call(b200s_plan* p, cudaStream_t st, bool capturing) {
-    if (p->used && p->last_stream != st && !capturing) {
-        const cudaError_t e = cudaStreamWaitEvent(st, p->done, 0);
-        if (e != cudaSuccess) return cuda_error(e, "plan order");
-    }
-    return B200S_OK;
+// for that one's end.  Streams are told apart by their ids, which are unique for
+// the program's life: one handle can name two streams (cudaStreamPerThread in
+// two host threads, a handle reused after its stream was destroyed).  Inside a
+// stream capture the order is the caller's.
+b200s_status begin_call(b200s_plan* p, cudaStream_t st, bool capturing, unsigned long long* id) {
+    *id = 0;
+    if (capturing) return B200S_OK;
+    cudaError_t e = cudaStreamGetId(st, id);
+    if (e == cudaSuccess && p->used && p->last_stream != *id) e = cudaStreamWaitEvent(st, p->done, 0);
+    return e == cudaSuccess ? B200S_OK : cuda_error(e, "plan order");
 }
-b200s_status end_call(b200s_plan* p, cudaStream_t st, bool capturing) {
+b200s_status end_call(b200s_plan* p, cudaStream_t st, bool capturing, unsigned long long id) {
     if (capturing) return B200S_OK;
     const cudaError_t e = cudaEventRecord(p->done, st);
     if (e != cudaSuccess) return cuda_error(e, "plan order");
-    p->last_stream = st;
+    p->last_stream = id;
     p->used = true;
     return B200S_OK;
 }
@@ -318,9 +321,10 @@ b200s_status is_capturing(cudaStream_t st, bool* out) {
 b200s_status run_direct(b200s_plan* p, const void* in, void* out, const int* off, int arrays, cudaStream_t st,
                         bool capturing, uint32_t present = ~0u, uint32_t over_present = ~0u,
                         const int* over_count = nullptr) {
-    b200s_status s = begin_call(p, st, capturing);
+    unsigned long long id = 0;
+    b200s_status s = begin_call(p, st, capturing, &id);
     if (s == B200S_OK) s = record_sequence(p, in, out, off, arrays, st, present, over_present, over_count);
-    if (s == B200S_OK) s = end_call(p, st, capturing);
+    if (s == B200S_OK) s = end_call(p, st, capturing, id);
     return s;
 }
 
@@ -493,10 +497,11 @@ b200s_status b200s_sort_ragged(b200s_plan* p, const void* d_in, void* d_out, con
         }
         p->graph_call = call;
     }
-    if ((status = begin_call(p, st, false)) != B200S_OK) return status;
+    unsigned long long id = 0;
+    if ((status = begin_call(p, st, false, &id)) != B200S_OK) return status;
     e = cudaGraphLaunch(p->exec, st);
     if (e != cudaSuccess) return cuda_error(e, "graph launch");
-    return end_call(p, st, false);
+    return end_call(p, st, false, id);
 }
 
 b200s_status b200s_sort_ragged_hinted(b200s_plan* p, const void* d_in, void* d_out, const int32_t* d_offsets,
