@@ -401,8 +401,8 @@ const std::vector<PassesEntry>& passes_registry() {
 // tile then, which needs no passes.  Measured, passes / tile (us): one array of
 // 8000 records 14.1 / 18.3, 30000 23.9 / 42.3, 65536 30.6 / 59.5; 16 arrays of
 // 65536 53 / 83; 64 of 16000 27.8 / 27.7 and 128 of them 45.5 / 43.1 (tile).
-// Not for stable records (no room for positions between passes), buffers that
-// are only 4-byte aligned, and the sortedness check of single-CTA tiles.
+// Not for stable records (no room for positions between passes), an output that
+// is not aligned to the record, and the sortedness check of single-CTA tiles.
 const PassesEntry* passes_for(int dtype, int stable, const void* out, int n, long long arrays, unsigned opts) {
     const int logw = ceil_log2(n);
     if (stable || (reinterpret_cast<uintptr_t>(out) % elem_bytes(dtype)) != 0) return nullptr;

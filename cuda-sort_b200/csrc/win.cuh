@@ -192,13 +192,25 @@ struct Win {
     // elements) with coalesced accesses through the region, in the layout kIo,
     // so that only the warp has to synchronise.  `first`: index of the tile's
     // element 0 in the array of n; elements at or beyond n are padding.
-    // A record buffer that is only 4-byte aligned moves word by word.
+    // A record buffer that is not aligned to the record moves element by
+    // element, 16-byte records word by word in a loop, which keeps that path's
+    // code short.
     static __device__ __forceinline__ int io_index(const int t) { return (t & 31) | ((t >> 5) << (LK + 5)); }
+    static constexpr bool kWords = sizeof(typename E::Mem) == 16;
+    static __device__ __forceinline__ int io_offset(const int q) {
+        int a = 0;
+        sfor<0, LK>([&](auto rc) {
+            constexpr int r = decltype(rc)::value;
+            constexpr int wt = P::kT.weight[P::kT.io.reg[r]];
+            a += ((q >> r) & 1) * wt;
+        });
+        return a;
+    }
 
     // Load into the natural layout.  pay: the payloads by position (gathered types).
     static __device__ __forceinline__ void load(R (&v)[K], const typename E::Mem* src, const int t, const int first,
                                                 const int n, R* sm, int32_t* pay = nullptr) {
-        if (!xp_wide(src)) {  // uniform: natural loads, and the region's padding
+        if (!kWords && !xp_wide(src)) {  // uniform: natural loads, and the region's padding
             const int i0 = rank(t) * K;
             load_tile<E, K>(v, src, first + i0, n);
             if constexpr (gathers<E>::value)
@@ -212,20 +224,30 @@ struct Win {
         // without a branch: a store inside the bounds test kept the loads of
         // gathered types apart (4 M stable records, W = 1024 / 2048 / 4096:
         // 68.6 / 76.7 / 83.3 -> 57.6 / 67.0 / 76.7 us).
-        typename E::Mem m[K];
-        sfor<0, K>([&](auto qc) {
-            constexpr int q = decltype(qc)::value;
-            const int idx = first + i0 + 32 * q;
-            if (idx < n) m[q] = xp_ldcs(src + idx);
-        });
-        sfor<0, K>([&](auto qc) {
-            constexpr int q = decltype(qc)::value;
-            constexpr int off = P::reg_off(P::kT.io, q);
-            const int i = i0 + 32 * q, idx = first + i;
-            if constexpr (gathers<E>::value)
-                if (pay) pay[i] = m[q].data;
-            sh_st(&sm[b + off], idx < n ? E::from_mem(m[q], idx) : E::pad());
-        });
+        if (kWords && !xp_wide(src)) {
+            if constexpr (kWords) {
+#pragma unroll 1
+                for (int q = 0; q < K; ++q) {
+                    const int idx = first + i0 + 32 * q;
+                    sh_st(&sm[b + io_offset(q)], idx < n ? E::from_mem(xp_ld_words(src + idx), idx) : E::pad());
+                }
+            }
+        } else {
+            typename E::Mem m[K];
+            sfor<0, K>([&](auto qc) {
+                constexpr int q = decltype(qc)::value;
+                const int idx = first + i0 + 32 * q;
+                if (idx < n) m[q] = xp_ldcs(src + idx);
+            });
+            sfor<0, K>([&](auto qc) {
+                constexpr int q = decltype(qc)::value;
+                constexpr int off = P::reg_off(P::kT.io, q);
+                const int i = i0 + 32 * q, idx = first + i;
+                if constexpr (gathers<E>::value)
+                    if (pay) pay[i] = m[q].data;
+                sh_st(&sm[b + off], idx < n ? E::from_mem(m[q], idx) : E::pad());
+            });
+        }
         __syncwarp();
         get<0>(v, t, sm);
     }
@@ -243,13 +265,23 @@ struct Win {
     static __device__ __forceinline__ void store(const R (&v)[K], typename E::Mem* dst, const int t, const int first,
                                                  const int n, R* sm) {
         if (dead(t, n - first)) return;
-        if (!xp_wide(dst)) {
+        if (!kWords && !xp_wide(dst)) {
             store_tile<E, K>(v, dst, first + rank(t) * K, n);
             return;
         }
         put<0>(v, t, sm);
         __syncwarp();
         const int i0 = io_index(t), b = base<kIo, false>(t);
+        if (kWords && !xp_wide(dst)) {
+            if constexpr (kWords) {
+#pragma unroll 1
+                for (int q = 0; q < K; ++q) {
+                    const int idx = first + i0 + 32 * q;
+                    if (idx < n) xp_st_words(dst + idx, E::to_mem(sh_ld(&sm[b + io_offset(q)])));
+                }
+            }
+            return;
+        }
         sfor<0, K>([&](auto qc) {
             constexpr int q = decltype(qc)::value;
             constexpr int off = P::reg_off(P::kT.io, q);

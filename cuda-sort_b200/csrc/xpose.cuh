@@ -116,10 +116,28 @@ __device__ __forceinline__ void xp_st(RecU64* p, const RecU64& v) {
 }
 
 // Whether whole-element accesses of p are aligned (always, but for records in
-// a buffer that is only 4-byte aligned).
+// a buffer that is not aligned to the record).
 template <class M>
 __device__ __forceinline__ bool xp_wide(const M* p) {
-    return sizeof(M) != 8 || (reinterpret_cast<uintptr_t>(p) & 7u) == 0;
+    return sizeof(M) < 8 || (reinterpret_cast<uintptr_t>(p) & (sizeof(M) - 1)) == 0;
+}
+
+// 16-byte records by words, for such buffers (the type itself promises its
+// alignment, so that an access to the whole record may be a 128-bit one).
+__device__ __forceinline__ RecU64 xp_ld_words(const RecU64* p) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(p);
+    RecU64 m;
+    from_u4<0>(make_uint4(w[0], w[1], w[2], w[3]), m);
+    return m;
+}
+__device__ __forceinline__ void xp_st_words(RecU64* p, const RecU64& v) {
+    uint4 u;
+    to_u4<0>(u, v);
+    uint32_t* w = reinterpret_cast<uint32_t*>(p);
+    w[0] = u.x;
+    w[1] = u.y;
+    w[2] = u.z;
+    w[3] = u.w;
 }
 
 // Element types whose tie order cannot be observed (keys alone: equal keys

@@ -159,7 +159,7 @@ b200s_status b200s_load_tile_table(const char* path, int32_t* applied);
  * than one CTA holds and for small batches of arrays beyond 4096 elements, a
  * sort in passes: one launch for slices of the arrays and two per later stage
  * of the network, in place in d_out, with the same output (not for stable
- * records, nor for record buffers that are only 4-byte aligned).  The single-CTA
+ * records, nor into a record buffer that is not aligned to the record).  The single-CTA
  * launches and the passes allow programmatic stream serialization: their CTAs may be
  * scheduled while the stream's previous kernel drains, and each waits for
  * that kernel's completion (griddepcontrol.wait) before touching memory, so
