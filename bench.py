@@ -645,7 +645,9 @@ def run_gpu(args, wl):
             form = t.persistent if args.form == "table" else int(args.form)
             tile = bs.Tile(shape[0], shape[1], shape[2], 0, form, 0 if args.tile else t.log2_ctas)
         eff = tile if tile is not None else bs.default_tile(dtype, n, flags)
-        extra["tile"] = repr(eff)
+        slice_bits = bs.packed_slice(dtype, n, arrays, flags) if tile is None else 0
+        passes = slice_bits > 0
+        extra["tile"] = "in passes, slices of %d" % (1 << slice_bits) if passes else repr(eff)
         tma_ok = (n * eb) % 128 == 0 and n * eb // 128 <= 256 and eff.log2_warps == 0 and eff.log2_ctas == 0
         form = eff.persistent if (eff.persistent != 2 or tma_ok) else 0
 
@@ -662,12 +664,9 @@ def run_gpu(args, wl):
         cluster = info.arrays_per_cta == 0
         if form == 3 and not info.xpose_form:
             form = 0
-        # arrays beyond one CTA without a tile request are sorted in passes (one
-        # launch for the slices, two per stage above them); the tile's CTA
-        # bits count the stages only when the tile was asked for
-        passes = cluster and tile is None and not (flags & bs.STABLE)
-        slice_bits = 13 if dtype == bs.U64_I32 else 14
-        stages = max(0, int(n - 1).bit_length() - slice_bits) if passes else 0
+        # in passes: one launch for the slices, two per stage above them; the
+        # tile's CTA bits count the stages only when the tile was asked for
+        stages = int(n - 1).bit_length() - slice_bits if passes else 0
         if passes:
             kernel = "k_sort_slices, k_merge_far, k_merge_near"
         elif form == 3:

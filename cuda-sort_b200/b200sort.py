@@ -199,6 +199,13 @@ def default_tile(dtype, n, flags=0):
     return t
 
 
+def packed_slice(dtype, n, arrays, flags=0):
+    """log2 of the slice length when sort_packed without a tile sorts the batch in passes, else 0."""
+    fn = declare("b200s_internal_packed_slice", ctypes.c_int32, [ctypes.c_int, ctypes.c_uint32, ctypes.c_int32,
+                                                                 ctypes.c_int64])
+    return fn(dtype, flags, n, arrays)
+
+
 def tile_info(dtype, n, flags=0, tile=None):
     """Registers, local memory, shared memory and residency of the kernel for length n."""
     out = TileInfo()

@@ -93,6 +93,9 @@ constexpr int kMaxLog2W = 20;
 struct DefaultTable {
     int pick[4][2][kMaxLog2W + 1];        // registry index, -1 if none
     int persistent[4][2][kMaxLog2W + 1];  // launch form for that row
+    // whether a batch of that length may be sorted in passes instead (passes_for);
+    // a row that does not say so is run as it stands, for every batch size
+    bool passes[4][2][kMaxLog2W + 1];
 };
 
 std::mutex g_table_mutex;
@@ -122,12 +125,13 @@ DefaultTable build_defaults() {
                 }
                 t.pick[d][s][w] = best;
                 t.persistent[d][s][w] = 0;
+                t.passes[d][s][w] = true;
             }
     return t;
 }
 
 struct TableRows {
-    std::vector<std::array<int, 4>> packed;  // dtype*2+stable, log2w, registry index, persistent
+    std::vector<std::array<int, 5>> packed;  // dtype*2+stable, log2w, registry index, persistent, passes
     std::vector<std::array<int, 6>> ragged;  // dtype, stable, log2w, family, own tile (registry index or -1), form
 };
 b200s_status parse_table_file(const char* path, TableRows* out);
@@ -157,12 +161,13 @@ DefaultTable& table() {
 
 // Entry for arrays of length n: the tabled tile for the smallest compiled
 // working length >= n.
-int lookup_default(int dtype, int stable, long long n, int* persistent) {
+int lookup_default(int dtype, int stable, long long n, int* persistent, bool* passes = nullptr) {
     std::lock_guard<std::mutex> lock(g_table_mutex);
     const DefaultTable& t = table();
     for (int w = std::max(0, ceil_log2(n)); w <= kMaxLog2W; ++w)
         if (t.pick[dtype][stable][w] >= 0) {
             *persistent = t.persistent[dtype][stable][w];
+            if (passes) *passes = t.passes[dtype][stable][w];
             return t.pick[dtype][stable][w];
         }
     return -1;
@@ -195,7 +200,7 @@ bool valid_dtype(int d) { return d >= 0 && d <= 3; }
 namespace {
 
 // Tile table CSV: '#' comments; packed rows dtype,flags,log2_w,log2_items,
-// log2_lanes,log2_warps[,persistent[,log2_ctas]]; ragged rows
+// log2_lanes,log2_warps[,persistent[,log2_ctas[,passes]]]; ragged rows
 // r,dtype,flags,log2_w,family.
 b200s_status parse_table_file(const char* path, TableRows* out) {
     std::ifstream f(path);
@@ -232,12 +237,13 @@ b200s_status parse_table_file(const char* path, TableRows* out) {
             out->ragged.push_back({d, stable, w, fam, own, form});
             continue;
         }
-        int d, fl, w, lk, lg, lw, pers = 0, lc = 0;
+        int d, fl, w, lk, lg, lw, pers = 0, lc = 0, passes = 0;
         if (!(ss >> d >> fl >> w >> lk >> lg >> lw))
             return set_error(B200S_ERR_INVALID_ARGUMENT,
-                             "tile table line " + std::to_string(lineno) + ": expected 6 to 8 integers");
+                             "tile table line " + std::to_string(lineno) + ": expected 6 to 9 integers");
         if (!(ss >> pers)) pers = 0;
         else if (!(ss >> lc)) lc = 0;
+        else if (!(ss >> passes)) passes = 0;
         if (!valid_dtype(d) || w < 0 || w > kMaxLog2W)
             return set_error(B200S_ERR_INVALID_ARGUMENT,
                              "tile table line " + std::to_string(lineno) + ": bad dtype or log2_w");
@@ -250,7 +256,10 @@ b200s_status parse_table_file(const char* path, TableRows* out) {
         if (pers < 0 || pers > 3)
             return set_error(B200S_ERR_INVALID_ARGUMENT,
                              "tile table line " + std::to_string(lineno) + ": launch form must be 0 .. 3");
-        out->packed.push_back({d * 2 + stable, w, idx, pers});
+        if (passes != 0 && passes != 1)
+            return set_error(B200S_ERR_INVALID_ARGUMENT,
+                             "tile table line " + std::to_string(lineno) + ": passes must be 0 or 1");
+        out->packed.push_back({d * 2 + stable, w, idx, pers, passes});
     }
     return B200S_OK;
 }
@@ -259,6 +268,7 @@ void apply_packed_rows(const TableRows& rows, DefaultTable& t) {
     for (const auto& u : rows.packed) {
         t.pick[u[0] / 2][u[0] % 2][u[1]] = u[2];
         t.persistent[u[0] / 2][u[0] % 2][u[1]] = u[3];
+        t.passes[u[0] / 2][u[0] % 2][u[1]] = u[4] != 0;
     }
 }
 
@@ -394,7 +404,8 @@ const std::vector<PassesEntry>& passes_registry() {
     return all;
 }
 
-// The sort in passes (passes.cuh) for a batch without a tile request, or null.
+// The sort in passes (passes.cuh) for a batch without a tile request whose
+// table row allows it, or null.
 // The smallest slices that number at most one per SM: more CTAs per array than
 // a single-CTA or cluster tile has, and none waits for another.  A batch of
 // more slices takes the largest ones; an array that one CTA holds goes to its
@@ -421,11 +432,12 @@ const PassesEntry* passes_for(int dtype, int stable, const void* out, int n, lon
     return last;
 }
 
-// launch_packed for a batch without a tile request.
-b200s_status launch_default(int idx, int persistent, const void* in, void* out, int n, long long arrays,
+// launch_packed for a batch without a tile request; passes: its table row
+// allows the sort in passes.
+b200s_status launch_default(int idx, int persistent, bool passes, const void* in, void* out, int n, long long arrays,
                             cudaStream_t st, unsigned opts) {
     const KernelEntry& e = registry()[size_t(idx)];
-    if (arrays < (1LL << 40))
+    if (passes && arrays < (1LL << 40))
         if (const PassesEntry* p = passes_for(e.dtype, e.stable, out, n, arrays, opts)) {
             const cudaError_t err = p->launch(in, out, n, arrays, ceil_log2(n), st);
             return err == cudaSuccess ? B200S_OK : cuda_error(err, "sort in passes");
@@ -434,10 +446,11 @@ b200s_status launch_default(int idx, int persistent, const void* in, void* out, 
 }
 
 int select_entry(int dtype, uint32_t flags, long long n, const b200s_tile* tile, b200s_status* st,
-                 int* persistent, long long arrays = -1) {
+                 int* persistent, long long arrays = -1, bool* passes = nullptr) {
     const int stable = effective_stable(dtype, flags);
     int idx;
     *persistent = 0;
+    if (passes) *passes = false;  // a requested tile is run as requested
     if (tile) {
         *persistent = tile->persistent < 0 ? 0 : (tile->persistent > 3 ? 3 : tile->persistent);
         idx = lookup_tile(dtype, stable, *tile);
@@ -450,7 +463,7 @@ int select_entry(int dtype, uint32_t flags, long long n, const b200s_tile* tile,
             return -1;
         }
     } else {
-        idx = lookup_default(dtype, stable, n, persistent);
+        idx = lookup_default(dtype, stable, n, persistent, passes);
         if (idx < 0) {
             *st = set_error(B200S_ERR_UNSUPPORTED, "array length exceeds the largest compiled tile");
             return -1;
@@ -611,11 +624,27 @@ b200s_status b200s_sort_packed(b200s_dtype dtype, const void* d_in, void* d_out,
     if (!d_in || !d_out) return set_error(B200S_ERR_INVALID_ARGUMENT, "null buffer");
     b200s_status st;
     int persistent = 0;
-    const int idx = select_entry(dtype, flags, n, tile, &st, &persistent, arrays);
+    bool passes = false;
+    const int idx = select_entry(dtype, flags, n, tile, &st, &persistent, arrays, &passes);
     if (idx < 0) return st;
-    return (tile ? launch_packed : launch_default)(idx, persistent, d_in, d_out, n, arrays,
-                                                   static_cast<cudaStream_t>(stream),
-                                                   (flags & B200S_SORTED_CHECK) ? kOptSortedCheck : 0u);
+    return launch_default(idx, persistent, passes, d_in, d_out, n, arrays, static_cast<cudaStream_t>(stream),
+                          (flags & B200S_SORTED_CHECK) ? kOptSortedCheck : 0u);
+}
+
+// For the bench, the tuner and the tests (not part of the C header): log2 of
+// the slice length when b200s_sort_packed without a tile sorts such a batch
+// (element-aligned buffers) in passes, 0 when it runs the tile, -1 on a bad
+// argument.
+int32_t b200s_internal_packed_slice(b200s_dtype dtype, uint32_t flags, int32_t n, int64_t arrays) {
+    if (!valid_dtype(dtype) || n <= 0 || arrays <= 0) return -1;
+    b200s_status st;
+    int persistent = 0;
+    bool passes = false;
+    if (select_entry(dtype, flags, n, nullptr, &st, &persistent, arrays, &passes) < 0) return -1;
+    const PassesEntry* p = passes ? passes_for(dtype, effective_stable(dtype, flags), nullptr, n, arrays,
+                                               (flags & B200S_SORTED_CHECK) ? kOptSortedCheck : 0u)
+                                  : nullptr;
+    return p ? p->log2_slice : 0;
 }
 
 }  // extern "C"
@@ -700,7 +729,8 @@ b200s_status b200s_sort_packed_host(b200s_session* s, b200s_dtype dtype, const v
     if (!h_in || !h_out) return set_error(B200S_ERR_INVALID_ARGUMENT, "null buffer");
     b200s_status st;
     int persistent = 0;
-    const int idx = select_entry(dtype, flags, n, nullptr, &st, &persistent);
+    bool passes = false;
+    const int idx = select_entry(dtype, flags, n, nullptr, &st, &persistent, -1, &passes);
     if (idx < 0) return st;
     cudaError_t e = cudaSetDevice(s->device);
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
@@ -749,7 +779,7 @@ b200s_status b200s_sort_packed_host(b200s_session* s, b200s_dtype dtype, const v
         if (e != cudaSuccess) return drain(cuda_error(e, "session slot wait"));
         e = cudaMemcpyAsync(s->dbuf[k], src + size_t(first) * array_bytes, bytes, cudaMemcpyHostToDevice, s->in);
         if (e != cudaSuccess) return drain(cuda_error(e, "host-to-device copy"));
-        st = launch_default(idx, persistent, s->dbuf[k], s->dbuf[k], n, count, s->in,
+        st = launch_default(idx, persistent, passes, s->dbuf[k], s->dbuf[k], n, count, s->in,
                             (flags & B200S_SORTED_CHECK) ? kOptSortedCheck : 0u);
         if (st != B200S_OK) return drain(st);
         e = cudaEventRecord(s->sorted[k], s->in);

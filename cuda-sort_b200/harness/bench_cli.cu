@@ -49,6 +49,8 @@
 
 #include "b200sort.h"
 
+// internal to libb200sort.so (see capi.cu)
+extern "C" int32_t b200s_internal_packed_slice(b200s_dtype dtype, uint32_t flags, int32_t n, int64_t arrays);
 extern "C" int cub_block_merge_sort(int dtype, void* d, int n, int arrays, int working, int threads, void* stream);
 extern "C" int thrust_segment_sort(int dtype, void* d, int n, int arrays, void* stream);
 
@@ -376,7 +378,8 @@ std::string tile_name(const b200s_tile& t) {
     return s.str();
 }
 
-template <class T> Config b200_config(const std::string& method, int n, const b200s_tile* tile) {
+// arrays: of the batch, which the sort in passes depends on (no tile given).
+template <class T> Config b200_config(const std::string& method, int n, const b200s_tile* tile, int arrays) {
     Config c;
     c.method = method;
     b200s_tile t;
@@ -391,7 +394,8 @@ template <class T> Config b200_config(const std::string& method, int n, const b2
     c.regs = info.registers_per_thread;
     c.active = info.active_ctas_per_sm;
     c.local = info.local_bytes_per_thread;
-    c.tile = tile_name(t);
+    const int slice = tile ? 0 : b200s_internal_packed_slice(dtype_of<T>(), 0, n, arrays);
+    c.tile = slice > 0 ? "passes/" + std::to_string(1 << slice) : tile_name(t);
     return c;
 }
 
@@ -414,14 +418,14 @@ template <class T> int reference_capacity() { return std::is_same<T, Rec>::value
 template <class T> void small_methods(Batch<T>& b, const Options& o) {
     const int n = b.n;
     if (o.enabled("b200_bitonic")) {
-        const Config c = b200_config<T>("b200_bitonic", n, nullptr);
+        const Config c = b200_config<T>("b200_bitonic", n, nullptr, b.arrays);
         b.run(c, [&] { return sort_b200(b, nullptr); });
     }
     for (const std::string& m : kLegacy) {
         if (!o.explicitly(m.c_str())) continue;
         if (m == "bitonic_warp" && n > 32) continue;
         if (m != "bitonic_warp" && n < 32) continue;
-        const Config c = b200_config<T>(m, n, nullptr);
+        const Config c = b200_config<T>(m, n, nullptr, b.arrays);
         b.run(c, [&] { return sort_b200(b, nullptr); });
     }
     if (o.enabled("b200_tiles")) {
@@ -434,7 +438,7 @@ template <class T> void small_methods(Batch<T>& b, const Options& o) {
             for (int pf = 0; pf < 2; ++pf) {
                 if (pf && t.log2_ctas) continue;
                 t.persistent = pf;
-                const Config c = b200_config<T>("b200_tiles", n, &t);
+                const Config c = b200_config<T>("b200_tiles", n, &t, b.arrays);
                 b.run(c, [&] { return sort_b200(b, &t); });
             }
         }
@@ -540,7 +544,7 @@ template <class T> void run_large(const Options& o, const std::string& type) {
             for (const std::string& m : kLarge) {
                 if (!o.enabled(m.c_str())) continue;
                 if (o.methods.empty() && m != "large_merge") continue;  // one row set by default
-                const Config c = b200_config<T>(m, n, nullptr);
+                const Config c = b200_config<T>(m, n, nullptr, b.arrays);
                 b.run(c, [&] { return sort_b200(b, nullptr); });
             }
             if (o.enabled("thrust_segment_loop")) {

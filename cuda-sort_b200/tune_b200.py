@@ -7,7 +7,9 @@ For every element type, stable flag and working length W = 2^L it times each
 compiled tile of that W (single-CTA and cluster tiles) in each launch form it
 has (0 one slot per array, 1 persistent with register prefetch, 2 persistent
 TMA pipeline, 3 transposed network) on a full-length batch of about 4 M
-elements, checks the output, and keeps the fastest as the packed row.  For the ragged kernel it
+elements, checks the output, and keeps the fastest as the packed row.  A row of a length
+that the library can sort in passes allows it, unless a full batch takes
+passes and they are slower than the fastest tile.  For the ragged kernel it
 times, per bucket L, a batch whose lengths all fall in that bucket in the
 persistent kernel with the bucket's shape family A, with family B, and as a
 launch of its own (the tabled tile of its working length, beside the
@@ -48,7 +50,7 @@ def _keys(dtype, arr):
     return arr if dtype in (bs.I32, bs.U64) else arr["key"]
 
 
-def tune_packed(dtype, flags, flush, passes, log, summary):
+def tune_packed(dtype, flags, flush, passes_per_row, log, summary):
     rows = []
     tiles = [t for t in bs.tiles(dtype, flags) if t.cta_threads > 0]   # single-CTA and cluster tiles
     by_w = {}
@@ -75,7 +77,7 @@ def tune_packed(dtype, flags, flush, passes, log, summary):
         for tile in cands:
             launches = [lambda i=i, t=tile: bs.sort_packed_status(dtype, ins[i].data_ptr(), outs[i].data_ptr(), n,
                                                                   arrays, flags, t, st) for i in range(sets)]
-            us, spread = devtime.batched_us(launches, flush, passes)
+            us, spread = devtime.batched_us(launches, flush, passes_per_row)
             if us is None:
                 continue
             ok = bool(np.array_equal(_keys(dtype, outs[0].cpu().numpy().view(bs.NP_DTYPES[dtype])), want))
@@ -87,21 +89,34 @@ def tune_packed(dtype, flags, flush, passes, log, summary):
         (us, spread, t) = results[0]
         second = results[1] if len(results) > 1 else None
         tail = (", runner-up %.2f us %s" % (second[0], _shape(second[2]))) if second else ""
-        lc = (",%d" % t.log2_ctas) if t.log2_ctas else ""
-        rows.append("%d,%d,%d,%d,%d,%d,%d%s  # %.2f us (spread %.1f %%)%s, %d arrays"
-                    % (dtype, flags, L, t.log2_items, t.log2_lanes, t.log2_warps, t.persistent, lc, us, 100 * spread,
-                       tail, arrays))
+        row = "%d,%d,%d,%d,%d,%d,%d,%d" % (dtype, flags, L, t.log2_items, t.log2_lanes, t.log2_warps, t.persistent,
+                                           t.log2_ctas)
+        load_rows([row + ",1"])
+        passes = bs.packed_slice(dtype, n, 1, flags) > 0
+        if passes and bs.packed_slice(dtype, n, arrays, flags) > 0:
+            passes_us, _ = devtime.batched_us([lambda i=i: bs.sort_packed_status(
+                dtype, ins[i].data_ptr(), outs[i].data_ptr(), n, arrays, flags, None, st) for i in range(sets)],
+                flush, passes_per_row)
+            log("packed dtype=%d flags=%d W=%d in passes: %.2f us" % (dtype, flags, n, passes_us))
+            passes = passes_us < us
+            tail += ", in passes %.2f us" % passes_us
+        rows.append("%s%s  # %.2f us (spread %.1f %%)%s, %d arrays"
+                    % (row, ",1" if passes else "", us, 100 * spread, tail, arrays))
         summary.append(("packed", dtype, flags, n, arrays, _shape(t), us, spread,
                         _shape(second[2]) if second else "-", second[0] if second else None))
         del ins, outs, src
         torch.cuda.empty_cache()
     # the ragged rows are timed with these packed rows in force (a launch of
     # its own runs the tabled tile in its tabled form)
+    load_rows(rows)
+    return rows
+
+
+def load_rows(rows):
     with tempfile.NamedTemporaryFile("w", suffix=".csv", delete=False) as f:
         f.write("\n".join(r.split("#")[0] for r in rows) + "\n")
     bs.load_tile_table(f.name)
     os.unlink(f.name)
-    return rows
 
 
 def _shape(t):
@@ -126,10 +141,7 @@ def tune_ragged(dtype, flags, flush, passes, log, summary):
         outs = [torch.empty_like(src) for _ in range(sets)]
         d_off = torch.from_numpy(off.astype(np.int32)).cuda()
         def time_row(row):
-            with tempfile.NamedTemporaryFile("w", suffix=".csv", delete=False) as f:
-                f.write(row + "\n")
-            bs.load_tile_table(f.name)
-            os.unlink(f.name)
+            load_rows([row])
             plans = [bs.Plan(dtype, arrays, flags) for _ in range(sets)]   # one captured graph per buffer set
             launches = [lambda i=i: plans[i].sort(ins[i].data_ptr(), outs[i].data_ptr(), d_off.data_ptr(), arrays, st)
                         for i in range(sets)]
@@ -175,11 +187,7 @@ def tune_ragged(dtype, flags, flush, passes, log, summary):
         del ins, outs, src
         torch.cuda.empty_cache()
         L += 1
-    # leave the process's table as tuned
-    with tempfile.NamedTemporaryFile("w", suffix=".csv", delete=False) as f:
-        f.write("\n".join(r.split("#")[0] for r in rows) + "\n")
-    bs.load_tile_table(f.name)
-    os.unlink(f.name)
+    load_rows(rows)   # leave the process's table as tuned
     return rows
 
 
@@ -221,8 +229,8 @@ def main():
         f.write("# device: %s; %s; library: %s\n" % (torch.cuda.get_device_name(),
                                                      datetime.datetime.now(datetime.timezone.utc).strftime(
                                                          "%Y-%m-%d %H:%M UTC"), bs.version()))
-        f.write("# packed rows: dtype,flags,log2_w,log2_items,log2_lanes,log2_warps,form (0 one-shot, 1 prefetch, 2 TMA, "
-                "3 transposed)\n")
+        f.write("# packed rows: dtype,flags,log2_w,log2_items,log2_lanes,log2_warps,form[,log2_ctas[,passes]] (form: 0 "
+                "one-shot, 1 prefetch, 2 TMA, 3 transposed; passes 1: batches may be sorted in passes instead)\n")
         f.write("# ragged rows: r,dtype,flags,log2_w,family[,log2_items,log2_lanes,log2_warps,form] (0: persistent, "
                 "larger per-thread tile; 1: persistent, smaller; 2: a launch of its own, in the tile and form given)\n")
         for ln in lines:

@@ -114,7 +114,10 @@ int32_t b200s_max_length(b200s_dtype dtype, uint32_t flags);
 /* Compiled tiles, for autotuning: index in [0, b200s_tile_count). */
 int32_t b200s_tile_count(b200s_dtype dtype, uint32_t flags);
 b200s_status b200s_tile_get(b200s_dtype dtype, uint32_t flags, int32_t index, b200s_tile* out);
-/* Tile the library uses for arrays of length n when the caller passes none. */
+/* Tile of the table for arrays of length n: what b200s_sort_packed without a
+ * tile runs, except for the batches that it sorts in passes or in a narrower
+ * cluster tile (see there), and what a ragged batch's cluster classes and
+ * launches of their own run. */
 b200s_status b200s_default_tile(b200s_dtype dtype, uint32_t flags, int32_t n, b200s_tile* out);
 /* Resources of the kernel that sorts arrays of length n with `tile` (NULL:
  * the default tile), as the reference's bench reports them for its kernels
@@ -145,8 +148,10 @@ b200s_status b200s_tma_timeouts(int64_t* count);
 b200s_status b200s_test_stall_tma_loads(int32_t enable);
 /* Replace rows of the default tile table from a CSV file; '#' starts a
  * comment.  Packed rows: dtype,flags,log2_w,log2_items,log2_lanes,log2_warps
- * [,form[,log2_ctas]] (form: 0 .. 3 as b200s_tile.persistent; log2_ctas: CTAs
- * per array of a cluster tile, default 0).  Ragged rows: r,dtype,flags,log2_w,family
+ * [,form[,log2_ctas[,passes]]] (form: 0 .. 3 as b200s_tile.persistent; log2_ctas: CTAs
+ * per array of a cluster tile, default 0; passes 1: b200s_sort_packed may sort batches
+ * of that length in passes instead, as the shipped rows say where that is faster; 0,
+ * the default: the row's tile sorts every batch).  Ragged rows: r,dtype,flags,log2_w,family
  * [,log2_items,log2_lanes,log2_warps,form] (0: the persistent kernel with the larger per-thread tile, 1: with
  * the smaller one, 2: a launch of its own, in the single-CTA tile and form (0 or 3) given, or without them the
  * packed table's tile and form for that length), read by plans created afterwards.
@@ -156,8 +161,8 @@ b200s_status b200s_load_tile_table(const char* path, int32_t* applied);
 /* Sort `arrays` independent arrays of n elements each, packed back to back
  * (array a at element offset a*n), from d_in into d_out (device pointers; may
  * be equal).  tile == NULL uses the default tile for n, or, for arrays longer
- * than one CTA holds and for small batches of arrays beyond 4096 elements, a
- * sort in passes: one launch for slices of the arrays and two per later stage
+ * than one CTA holds and for small batches of arrays beyond 4096 elements, if
+ * the length's table row allows it, a sort in passes: one launch for slices of the arrays and two per later stage
  * of the network, in place in d_out, with the same output (not for stable
  * records, nor into a record buffer that is not aligned to the record).  The single-CTA
  * launches and the passes allow programmatic stream serialization: their CTAs may be
