@@ -139,12 +139,16 @@ struct Packed {
     }
 };
 
-// A packed batch of at most this many warps runs the latency form of a tile
-// that has one (ElemRecI32L): four warps per SM.  Measured, default / latency
+// A packed batch of at most this many warps per SM runs the latency form of a
+// tile that has one (ElemRecI32L).  Measured on 148 SMs, default / latency
 // form (us): 60 arrays of 200 records 4.5 / 3.6, of 500 5.4 / 4.6, of 1000
 // 6.4 / 5.6, of 2000 7.4 / 6.3; 1200 arrays of 200 5.4 / 5.2, of 500 6.9 / 8.0,
 // 400 of 1000 7.2 / 7.2, of 2000 10.3 / 12.3.
-constexpr long long kLatencyWarps = 592;
+constexpr int kLatencyWarps = 4;
+template <class E, class LAT>
+bool latency_form(long long warps) {
+    return !std::is_same_v<E, LAT> && warps <= (long long)kLatencyWarps * sm_count();
+}
 
 // Opt in to SMEM bytes of dynamic shared memory for kernel fn (once per
 // device), with a margin for the kernel's own static variables.

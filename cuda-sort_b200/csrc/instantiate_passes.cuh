@@ -50,7 +50,7 @@ struct Passes {
             const Mem* src = static_cast<const Mem*>(in) + first * n;
             Mem* dst = static_cast<Mem*>(out) + first * n;
             const long long ctas = count << (logw - LOCAL);
-            const int early = ctas <= 64 || ctas >= 148 * (kSmThreads / S::TPA);  // see passes.cuh
+            const int early = ctas <= 64 || ctas >= (long long)sm_count() * (kSmThreads / S::TPA);  // see passes.cuh
             e = launch_pdl(slices, unsigned(ctas), S::TPA, SMEM, st, src, dst, n, logw - LOCAL, early);
             if (e == cudaSuccess) e = stages<LOCAL>(dst, n, count, logw, early, st);
         }

@@ -33,7 +33,7 @@ struct PackedXc {
     static cudaError_t launch(const void* in, void* out, int n, long long arrays, long long,
                               cudaStream_t st, unsigned opts) {
         if (opts & kOptSortedCheck) return launch_form<E, true>(in, out, n, arrays, st);
-        if (!std::is_same_v<E, LAT> && (arrays << LW) <= kLatencyWarps)
+        if (latency_form<E, LAT>(arrays << LW))
             return launch_form<LAT, false>(in, out, n, arrays, st);
         return launch_form<E, false>(in, out, n, arrays, st);
     }

@@ -613,7 +613,7 @@ b200s_status b200s_internal_check_offsets(const void* off, int32_t is64, int64_t
     if (!off || !d_flag || arrays < 0 || (is64 && !off32))
         return set_error(B200S_ERR_INVALID_ARGUMENT, "b200s_internal_check_offsets: bad argument");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const long long blocks = std::min<long long>((arrays + kCheckThreads) / kCheckThreads, 592);
+    const long long blocks = std::min<long long>((arrays + kCheckThreads) / kCheckThreads, 4LL * sm_count());
     cudaError_t e = blocks > 1 ? cudaMemsetAsync(d_flag, 0, sizeof(int32_t), st) : cudaSuccess;
     if (e == cudaSuccess) {
         if (is64)

@@ -71,6 +71,8 @@ void register_xc_u64rec(std::vector<KernelEntry>& out);
 
 const std::vector<KernelEntry>& registry();
 
+int sm_count();  // SMs of the current device (cached per device)
+
 struct RaggedCtl;
 
 // The persistent ragged kernel of one element type.
