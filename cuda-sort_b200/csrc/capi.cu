@@ -70,6 +70,7 @@ const std::vector<KernelEntry>& registry() {
         register_cluster_u64rec(v);
         register_xc_keys(v);
         register_xc_rec(v);
+        register_xc_rec_wide(v);
         register_xc_cluster_rec(v);
         register_xc_u64rec(v);
         // single-warp tiles: launch form 3 over id lists is the one-warp

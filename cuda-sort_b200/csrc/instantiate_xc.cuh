@@ -32,10 +32,11 @@ struct PackedXc {
     }
     static cudaError_t launch(const void* in, void* out, int n, long long arrays, long long,
                               cudaStream_t st, unsigned opts) {
-        if (opts & kOptSortedCheck) return launch_form<E, true>(in, out, n, arrays, st);
+        const bool check = (opts & kOptSortedCheck) != 0;
         if (latency_form<E, LAT>(arrays << LW))
-            return launch_form<LAT, false>(in, out, n, arrays, st);
-        return launch_form<E, false>(in, out, n, arrays, st);
+            return check ? launch_form<LAT, true>(in, out, n, arrays, st)
+                         : launch_form<LAT, false>(in, out, n, arrays, st);
+        return check ? launch_form<E, true>(in, out, n, arrays, st) : launch_form<E, false>(in, out, n, arrays, st);
     }
     static cudaError_t launch_list(const void* in, void* out, const int* off, const int* ids, int count,
                                    cudaStream_t st) {

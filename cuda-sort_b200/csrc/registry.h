@@ -66,6 +66,7 @@ void register_cluster_u64rec(std::vector<KernelEntry>& out);
 // above (run last).
 void register_xc_keys(std::vector<KernelEntry>& out);
 void register_xc_rec(std::vector<KernelEntry>& out);
+void register_xc_rec_wide(std::vector<KernelEntry>& out);
 void register_xc_cluster_rec(std::vector<KernelEntry>& out);
 void register_xc_u64rec(std::vector<KernelEntry>& out);
 

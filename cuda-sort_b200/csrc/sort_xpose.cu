@@ -38,7 +38,7 @@ struct Xpose {
         const long long grid = std::min<long long>((arrays + per_cta - 1) / per_cta, 0x7fffffffLL);
         const auto* src = static_cast<const typename E::Mem*>(in);
         auto* dst = static_cast<typename E::Mem*>(out);
-        if (latency_form<E, LAT>(grid * WPC) && !(opts & kOptSortedCheck))
+        if (latency_form<E, LAT>(grid * WPC))
             return launch_pdl(kernel<LAT>(), unsigned(grid), WPC * 32, SMEM, st, src, dst, n, arrays, opts);
         return launch_pdl(kernel(), unsigned(grid), WPC * 32, SMEM, st, src, dst, n, arrays, opts);
     }
