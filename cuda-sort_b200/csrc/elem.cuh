@@ -209,6 +209,21 @@ struct ElemU64 {
     }
 };
 
+// The same with compare and selects, the latency form of the tiles of W = 64 ..
+// 2048 (see ElemRecI32L).
+struct ElemU64L : ElemU64 {
+    template <int Q>
+    static __device__ __forceinline__ void cexq(Reg& lo, Reg& hi) {
+        cex(lo, hi);
+    }
+    static __device__ __forceinline__ void cex(Reg& lo, Reg& hi) {
+        const Reg a = lo, b = hi;
+        const bool sw = b < a;
+        lo = sw ? b : a;
+        hi = sw ? a : b;
+    }
+};
+
 // ---- records: int32 key + int32 payload (IntAndData) ------------------------
 struct RegRecI32 {
     int32_t key;

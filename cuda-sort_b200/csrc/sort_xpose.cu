@@ -106,9 +106,9 @@ const std::vector<XposeEntry>& xpose_registry() {
         constexpr int U64 = 2;                                     // B200S_U64
         v.push_back(Xpose<ElemU64, 5, 5, kXpIoStriped, 16>::entry(U64));    // W = 1024
         v.push_back(Xpose<ElemU64, 5, 4, kXpIoStriped, 16>::entry(U64));    // W = 512
-        v.push_back(Xpose<ElemU64, 4, 4, kXpIoStriped, 24>::entry(U64));    // W = 256
-        v.push_back(Xpose<ElemU64, 4, 3, kXpIoStriped, 24>::entry(U64));    // W = 128
-        v.push_back(Xpose<ElemU64, 4, 2, kXpIoStriped, 24>::entry(U64));    // W = 64
+        v.push_back(Xpose<ElemU64, 4, 4, kXpIoStriped, 24, ElemU64L>::entry(U64));    // W = 256
+        v.push_back(Xpose<ElemU64, 4, 3, kXpIoStriped, 24, ElemU64L>::entry(U64));    // W = 128
+        v.push_back(Xpose<ElemU64, 4, 2, kXpIoStriped, 24, ElemU64L>::entry(U64));    // W = 64
         return v;
     }();
     return all;

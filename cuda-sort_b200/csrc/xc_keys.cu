@@ -13,9 +13,9 @@ void register_xc_keys(std::vector<KernelEntry>& o) {
     ClusterXc<ElemI32, 5, 5, 4, 1, false>::attach_to(o, 0);
     ClusterXc<ElemI32, 5, 5, 4, 2, false>::attach_to(o, 0);
     ClusterXc<ElemI32, 5, 5, 4, 3, false>::attach_to(o, 0);
-    PackedXc<ElemU64, 4, 0, 32>::attach_to(o, 2);  // W = 512
-    PackedXc<ElemU64, 4, 1, 16>::attach_to(o, 2);
-    PackedXc<ElemU64, 4, 2, 8>::attach_to(o, 2);
+    PackedXc<ElemU64, 4, 0, 32, ElemU64L>::attach_to(o, 2);  // W = 512
+    PackedXc<ElemU64, 4, 1, 16, ElemU64L>::attach_to(o, 2);
+    PackedXc<ElemU64, 4, 2, 8, ElemU64L>::attach_to(o, 2);
     PackedXc<ElemU64, 4, 3, 4>::attach_to(o, 2);
     PackedXc<ElemU64, 4, 4, 2>::attach_to(o, 2);  // W = 8192
     ClusterXc<ElemU64, 4, 5, 5, 0, true>::attach_to(o, 2);
