@@ -7,7 +7,8 @@ For every element type, stable flag and working length W = 2^L it times each
 compiled tile of that W (single-CTA and cluster tiles) in each launch form it
 has (0 one slot per array, 1 persistent with register prefetch, 2 persistent
 TMA pipeline, 3 transposed network) on a full-length batch of about 4 M
-elements, checks the output, and keeps the fastest as the packed row.  A row of a length
+elements, checks the output, and keeps the fastest as the packed row, or one a
+little slower that is faster on a batch of a few arrays (pick_row).  A row of a length
 that the library can sort in passes allows it, unless a full batch takes
 passes and they are slower than the fastest tile.  For the ragged kernel it
 times, per bucket L, a batch whose lengths all fall in that bucket in the
@@ -44,6 +45,25 @@ FORM_NAMES = {0: "one-shot", 1: "prefetch", 2: "TMA", 3: "transposed"}
 # A / B; 2 gives the bucket a launch of its own, in the tile and form the row
 # names (the tuner searches them)
 FAMILY_NAMES = {0: "persistent A", 1: "persistent B", 2: "own launch"}
+
+
+# Full batches hide one array's latency and batches of a few arrays are all
+# latency, but a length has one row: a tile within NEAR of the fastest on the full
+# batch is kept when a batch of FEW arrays takes GAIN less time with it (more
+# threads per array, as a rule: int32 W = 2048 with 128 threads instead of 64 takes
+# 26.9 us instead of 25.5 per 4 M keys, and 3.7 instead of 5.3 for a few arrays).
+NEAR, FEW, GAIN = 1.06, 16, 0.95
+
+
+def pick_row(results, few_us):
+    """Index of the row among results, (us, spread, tile) with the fastest first;
+    few_us(tile): its time on a batch of FEW arrays."""
+    near = [i for i, r in enumerate(results) if r[0] <= NEAR * results[0][0]]
+    if len(near) == 1:
+        return 0
+    times = [few_us(results[i][2]) for i in near]
+    best = min(near, key=lambda i: times[i])
+    return best if times[best] <= GAIN * times[0] else 0
 
 
 def _keys(dtype, arr):
@@ -86,9 +106,16 @@ def tune_packed(dtype, flags, flush, passes_per_row, log, summary):
             if ok:
                 results.append((us, spread, tile))
         results.sort(key=lambda r: r[0])
-        (us, spread, t) = results[0]
-        second = results[1] if len(results) > 1 else None
-        tail = (", runner-up %.2f us %s" % (second[0], _shape(second[2]))) if second else ""
+
+        def few_us(tile):
+            return devtime.batched_us([lambda i=i: bs.sort_packed_status(dtype, ins[i].data_ptr(), outs[i].data_ptr(),
+                                                                         n, min(FEW, arrays), flags, tile, st)
+                                       for i in range(sets)], flush, passes_per_row)[0]
+
+        k = pick_row(results, few_us)
+        (us, spread, t) = results[k]
+        second = results[0] if k else results[1] if len(results) > 1 else None
+        tail = (", %s %.2f us %s" % ("kept over" if k else "runner-up", second[0], _shape(second[2]))) if second else ""
         row = "%d,%d,%d,%d,%d,%d,%d,%d" % (dtype, flags, L, t.log2_items, t.log2_lanes, t.log2_warps, t.persistent,
                                            t.log2_ctas)
         load_rows([row + ",1"])
@@ -229,6 +256,7 @@ def main():
         f.write("# device: %s; %s; library: %s\n" % (torch.cuda.get_device_name(),
                                                      datetime.datetime.now(datetime.timezone.utc).strftime(
                                                          "%Y-%m-%d %H:%M UTC"), bs.version()))
+        f.write("# rows \"kept over\" a faster full batch: the rule for batches of a few arrays (pick_row)\n")
         f.write("# packed rows: dtype,flags,log2_w,log2_items,log2_lanes,log2_warps,form[,log2_ctas[,passes]] (form: 0 "
                 "one-shot, 1 prefetch, 2 TMA, 3 transposed; passes 1: batches may be sorted in passes instead)\n")
         f.write("# ragged rows: r,dtype,flags,log2_w,family[,log2_items,log2_lanes,log2_warps,form] (0: persistent, "
