@@ -44,7 +44,6 @@ constexpr int kWinMaxWindows = 32;  // windows of one tile, the natural one incl
 
 struct WinClasses {
     int cls[kWinMaxBits];   // class of each index bit
-    int slot[3];            // classes of the bits that number a warp's arrays (tiles below a warp)
 };
 
 // Classes of the index bits for 2^LOGW-element tiles of 2^lk elements per
@@ -53,65 +52,54 @@ constexpr WinClasses win_classes(int lk, int logw, int m) {
     // 8-byte elements
     if (m == 4 && lk == 4) {
         switch (logw) {
-            case 5: return {{3, 0, 1, 2, 3}, {0, 1, 2}};
-            case 6: return {{3, 2, 3, 2, 3, 2}, {0, 1, 4}};
-            case 7: return {{1, 2, 1, 3, 1, 2, 3}, {0, 4, 4}};
-            case 8: return {{2, 1, 3, 0, 2, 1, 0, 3}, {4, 4, 4}};
-            case 9: return {{1, 3, 2, 0, 1, 3, 1, 2, 0}, {4, 4, 4}};
-            case 10: return {{0, 3, 2, 1, 0, 3, 0, 2, 1, 4}, {4, 4, 4}};
-            case 11: return {{0, 3, 2, 1, 0, 3, 0, 2, 1, 3, 1}, {4, 4, 4}};
-            case 12: return {{1, 0, 2, 1, 3, 0, 1, 2, 3, 1, 0, 4}, {4, 4, 4}};
-            case 13: return {{0, 1, 2, 3, 0, 1, 0, 2, 3, 4, 1, 3, 1}, {4, 4, 4}};
-            case 14: return {{0, 1, 2, 3, 0, 1, 0, 2, 3, 3, 1, 2, 2, 0}, {4, 4, 4}};
+            case 9: return {{1, 3, 2, 0, 1, 3, 1, 2, 0}};
+            case 10: return {{0, 3, 2, 1, 0, 3, 0, 2, 1, 4}};
+            case 11: return {{0, 3, 2, 1, 0, 3, 0, 2, 1, 3, 1}};
+            case 12: return {{1, 0, 2, 1, 3, 0, 1, 2, 3, 1, 0, 4}};
+            case 13: return {{0, 1, 2, 3, 0, 1, 0, 2, 3, 4, 1, 3, 1}};
+            case 14: return {{0, 1, 2, 3, 0, 1, 0, 2, 3, 3, 1, 2, 2, 0}};
         }
     }
     if (m == 4 && lk == 5) {
         switch (logw) {
-            case 6: return {{3, 4, 0, 3, 2, 3}, {0, 1, 2}};
-            case 7: return {{2, 3, 2, 2, 1, 2, 3}, {0, 1, 4}};
-            case 8: return {{1, 2, 3, 3, 2, 1, 3, 2}, {0, 4, 4}};
-            case 9: return {{2, 0, 2, 3, 1, 2, 0, 1, 3}, {4, 4, 4}};
-            case 10: return {{0, 3, 2, 1, 3, 3, 3, 1, 2, 0}, {4, 4, 4}};
-            case 11: return {{0, 3, 1, 3, 2, 3, 3, 2, 1, 0, 1}, {4, 4, 4}};
-            case 12: return {{0, 2, 1, 0, 3, 1, 1, 0, 2, 3, 3, 4}, {4, 4, 4}};
-            case 13: return {{2, 3, 0, 1, 2, 0, 3, 2, 1, 0, 0, 4, 2}, {4, 4, 4}};
-            case 14: return {{1, 2, 1, 3, 0, 1, 1, 2, 0, 3, 4, 0, 2, 3}, {4, 4, 4}};
+            case 11: return {{0, 3, 1, 3, 2, 3, 3, 2, 1, 0, 1}};
+            case 12: return {{0, 2, 1, 0, 3, 1, 1, 0, 2, 3, 3, 4}};
+            case 13: return {{2, 3, 0, 1, 2, 0, 3, 2, 1, 0, 0, 4, 2}};
         }
     }
     // 16-byte elements
     if (m == 3 && lk == 4) {
         switch (logw) {
-            case 9: return {{0, 1, 2, 0, 1, 1, 0, 0, 2}, {3, 3, 3}};
-            case 10: return {{0, 1, 2, 2, 0, 1, 0, 0, 2, 3}, {3, 3, 3}};
-            case 11: return {{1, 0, 2, 1, 0, 3, 0, 2, 1, 3, 2}, {3, 3, 3}};
-            case 12: return {{0, 0, 2, 0, 1, 1, 0, 2, 1, 0, 0, 0}, {3, 3, 3}};
-            case 13: return {{1, 1, 2, 0, 1, 1, 2, 0, 2, 3, 0, 0, 0}, {3, 3, 3}};
-            case 14: return {{1, 1, 2, 1, 0, 1, 0, 2, 0, 0, 1, 0, 1, 1}, {3, 3, 3}};
+            case 9: return {{0, 1, 2, 0, 1, 1, 0, 0, 2}};
+            case 10: return {{0, 1, 2, 2, 0, 1, 0, 0, 2, 3}};
+            case 11: return {{1, 0, 2, 1, 0, 3, 0, 2, 1, 3, 2}};
+            case 12: return {{0, 0, 2, 0, 1, 1, 0, 2, 1, 0, 0, 0}};
+            case 13: return {{1, 1, 2, 0, 1, 1, 2, 0, 2, 3, 0, 0, 0}};
+            case 14: return {{1, 1, 2, 1, 0, 1, 0, 2, 0, 0, 1, 0, 1, 1}};
         }
     }
     // 4-byte elements
     if (m == 5 && lk == 4) {
         switch (logw) {
-            case 9: return {{3, 1, 4, 2, 3, 1, 4, 2, 0}, {5, 5, 5}};
-            case 10: return {{0, 1, 2, 4, 0, 1, 2, 3, 4, 1}, {5, 5, 5}};
-            case 11: return {{4, 3, 1, 2, 4, 3, 2, 1, 0, 0, 4}, {5, 5, 5}};
-            case 12: return {{3, 1, 2, 0, 3, 1, 0, 2, 4, 0, 3, 1}, {5, 5, 5}};
-            case 13: return {{3, 1, 2, 0, 3, 1, 0, 2, 4, 4, 5, 2, 0}, {5, 5, 5}};
+            case 9: return {{3, 1, 4, 2, 3, 1, 4, 2, 0}};
+            case 10: return {{0, 1, 2, 4, 0, 1, 2, 3, 4, 1}};
+            case 11: return {{4, 3, 1, 2, 4, 3, 2, 1, 0, 0, 4}};
+            case 12: return {{3, 1, 2, 0, 3, 1, 0, 2, 4, 0, 3, 1}};
+            case 13: return {{3, 1, 2, 0, 3, 1, 0, 2, 4, 4, 5, 2, 0}};
         }
     }
     if (m == 5 && lk == 5) {
         switch (logw) {
-            case 10: return {{1, 4, 3, 0, 2, 1, 3, 0, 2, 4}, {5, 5, 5}};
-            case 11: return {{2, 3, 1, 4, 0, 2, 3, 0, 1, 4, 4}, {5, 5, 5}};
-            case 12: return {{1, 2, 0, 3, 4, 1, 2, 3, 0, 4, 3, 2}, {5, 5, 5}};
-            case 13: return {{0, 1, 4, 3, 2, 0, 1, 3, 2, 4, 5, 2, 0}, {5, 5, 5}};
-            case 14: return {{0, 3, 1, 4, 2, 0, 3, 2, 1, 4, 2, 4, 5, 5}, {5, 5, 5}};
+            case 10: return {{1, 4, 3, 0, 2, 1, 3, 0, 2, 4}};
+            case 11: return {{2, 3, 1, 4, 0, 2, 3, 0, 1, 4, 4}};
+            case 12: return {{1, 2, 0, 3, 4, 1, 2, 3, 0, 4, 3, 2}};
+            case 13: return {{0, 1, 4, 3, 2, 0, 1, 3, 2, 4, 5, 2, 0}};
+            case 14: return {{0, 3, 1, 4, 2, 0, 3, 2, 1, 4, 2, 4, 5, 5}};
         }
     }
     // no searched classes: the bits cycle through them
     WinClasses c{};
     for (int b = 0; b < kWinMaxBits; ++b) c.cls[b] = b % (m < lk ? m : lk);
-    for (int s = 0; s < 3; ++s) c.slot[s] = m;
     return c;
 }
 
@@ -125,8 +113,8 @@ struct WinLayout {
 
 template <int LK, int LOGW, int M>
 struct WinPlan {
-    static constexpr int LT = LOGW - LK, LG = LT < 5 ? LT : 5, LW = LT - LG;
-    static_assert(LOGW <= kWinMaxBits && LK >= 2 && LK <= 6, "tile shape");
+    static constexpr int LT = LOGW - LK, LG = 5, LW = LT - LG;
+    static_assert(LOGW <= kWinMaxBits && LK >= 2 && LK <= 6 && LT >= 5, "tile shape: whole warps");
     struct Tables {
         WinLayout win[kWinMaxWindows];  // [0]: natural
         WinLayout merge[6];             // windows of the merges on bits LOGW-1 .. 0 (after a cluster layer)
@@ -134,8 +122,8 @@ struct WinPlan {
         WinLayout io;                   // coalesced global accesses: lanes on the lowest index bits
         int windows;                    // windows after the natural one
         int weight[kWinMaxBits];        // shared-memory weight of each index bit
-        int slot[5];                    // and of each bit of the array's number inside a warp
-        int elems;                      // shared-memory elements of one warp's arrays (one array above a warp)
+        static constexpr int slot[5] = {};  // of the bits that number a warp's arrays: none, a tile is whole warps
+        int elems;                      // shared-memory elements of the tile
     };
 
     // Thread bits of a layout: the index bits left over, the lowest LG of them
@@ -213,11 +201,9 @@ struct WinPlan {
         t.io.refl = -1;
         for (int j = 0; j < LG; ++j) t.io.thr[j] = j;
         for (int j = LG; j < LT; ++j) t.io.thr[j] = LK + j;
-        // weights: index bits, then the slot bits
-        constexpr int N = LOGW + 5 - LG;
-        int cls[kWinMaxBits + 5] = {}, w[kWinMaxBits + 5] = {};
-        for (int b = 0; b < LOGW; ++b) cls[b] = c.cls[b];
-        for (int s = 0; s < 5 - LG; ++s) cls[LOGW + s] = s < 3 ? c.slot[s] : M;
+        // weights
+        int w[kWinMaxBits] = {};
+        const auto& cls = c.cls;
         int sum = 0;
         bool base = true;  // one bit of each class 0 .. M-1 among the index bits
         int first[8] = {};
@@ -244,16 +230,7 @@ struct WinPlan {
                     sum += v;
                 }
         }
-        for (int b = LOGW; b < N; ++b) {
-            const int k = cls[b];
-            const int mod = k == M ? 1 << M : 2 << k, want = k == M ? 0 : 1 << k;
-            int v = sum + 1;
-            while (v % mod != want) ++v;
-            w[b] = v;
-            sum += v;
-        }
         for (int b = 0; b < LOGW; ++b) t.weight[b] = w[b];
-        for (int s = 0; s < 5 - LG; ++s) t.slot[s] = w[LOGW + s];
         t.elems = sum + 1;
         return t;
     }
