@@ -378,7 +378,7 @@ int sm_count() {
 // leave SMs idle: on a 148-SM B200 (one 512-thread CTA per SM) 74 2-CTA, 33
 // 4-CTA and 15 8-CTA clusters are resident, i.e. 100 %, 89 % and 81 % of the
 // SMs; the rule allows arrays * CTAs per array up to that share.  One
-// 65536-record array: 60 us with 8 CTAs of 512 threads, 82 with 4 of 1024.
+// 65536-record array: 60 us with 8 CTAs of 512 threads, 87 with 4 of 1024.
 int narrow_alternative(int idx, long long arrays) {
     const auto& reg = registry();
     const KernelEntry& e = reg[size_t(idx)];
@@ -410,10 +410,10 @@ const std::vector<PassesEntry>& passes_registry() {
 // The smallest slices that number at most one per SM: more CTAs per array than
 // a single-CTA or cluster tile has, and none waits for another.  A batch of
 // more slices takes the largest ones; an array that one CTA holds goes to its
-// tile then, which needs no passes.  Measured, passes / tile (us): one array of
-// 8000 records 14.1 / 18.3, 30000 23.9 / 42.3, 65536 30.6 / 59.5; 16 arrays of
-// 65536 53 / 83; 64 of 16000 27.8 / 27.7 and 128 of them 45.5 / 43.1 (tile).
-// Not for stable records (no room for positions between passes), an output that
+// tile then, which needs no passes.  Measured, passes / fastest tile (us): one
+// array of 8000 records 14.5 / 18.8, 30000 28.3 / 43.1, 65536 35.7 / 59.8; 16 arrays
+// of 65536 60 / 87; 64 of 16000 29.3 / 29.1 (45.7 in the tabled tile).
+// Not for stable records (see passes.cuh), an output that
 // is not aligned to the record, and the sortedness check of single-CTA tiles.
 const PassesEntry* passes_for(int dtype, int stable, const void* out, int n, long long arrays, unsigned opts) {
     const int logw = ceil_log2(n);

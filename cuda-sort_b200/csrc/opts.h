@@ -3,8 +3,8 @@
 
 namespace b200s {
 
-// B200S_SORTED_CHECK: test each tile before sorting (and, in the transposed
-// network, after every stage of span >= 16) and skip the rest of the network
+// B200S_SORTED_CHECK: test each tile before sorting (and, in the one-warp
+// transposed network, after every stage of span >= 16) and skip the rest of the network
 // once it is in order, as the reference's Sorted switch does.
 constexpr unsigned kOptSortedCheck = 1u;
 

@@ -23,12 +23,13 @@
 // records and layer, and 4-CTA clusters leave 16 of 148 SMs idle; a pass moves
 // its 8 bytes in and out at HBM rate, about 10 us per 4 M records.  With few
 // arrays the passes win too: slices of 4096 spread one array over many SMs
-// (one array of 30000 records: 7 slices and 6 short passes take 24 us where
-// a cluster of four CTAs takes 42).  Measured against the clusters (us): 256
-// arrays of 65536 records 664 -> 480, 128 of 65536 uint64-key records
-// 1061 -> 598, 128 of 131072 int32 keys 482 -> 252.  The clusters stay for
-// ragged lists, whose counts only the device knows, and for stable records,
-// whose positions have no place in the output.
+// (one array of 30000 records: 8 slices and 6 short passes take 28 us where
+// a cluster of four CTAs takes 43).  Measured against the clusters (us): 256
+// arrays of 65536 records 688 -> 502, 128 of 65536 uint64-key records
+// 1064 -> 585, 128 of 131072 int32 keys 486 -> 256.  The clusters stay for
+// ragged lists, whose counts only the device knows, and for stable records:
+// their words need room between passes that a call in place does not have (out
+// of place a (key, position) word would fit the record's slot in the output).
 //
 // Programmatic dependent launch: each kernel waits for the one before it.  It
 // lets the next be scheduled at its start (`early`) when no grid can crowd

@@ -7,12 +7,13 @@
 // included, is the reference's.  Keys alone (kKeysOnly) sort each thread's
 // registers with Batcher's odd-even merge sort instead of stages 0 .. LK-1.
 //
-// What bounds it: at 16 elements per thread the shared-memory pipe (83 % of its
-// wavefronts at W = 4096 records) with the issue slots close behind (74 %);
-// the ALU and FMA pipes share the compare-exchanges (63 % each, elem.cuh).
+// What bounds it: at 16 elements per thread the shared-memory pipe (80 % of its
+// wavefronts at W = 4096 records) with the issue slots close behind (72 %);
+// the ALU and FMA pipes share the compare-exchanges (ALU 61 %, and 61 % of the
+// half of the FMA pipe that multiplies integers, elem.cuh).
 // 32 records per thread take a quarter fewer trips but their unrolled code
-// (100 KB and more) overflows the instruction cache: W = 1024 / 4096 / 8192 in
-// 41.6 / 57.7 / 73.0 us per 4 M records against 38.9 / 51.5 / 66.5 with 16.
+// (100 KB and more) overflows the instruction cache: W = 2048 / 4096 / 8192 in
+// 53.6 / 65.7 / 77.5 us per 4 M records against 47.6 / 53.9 / 66.9 with 16.
 #pragma once
 #include "win_layout.h"
 #include "xpose.cuh"

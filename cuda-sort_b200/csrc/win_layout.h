@@ -31,7 +31,8 @@
 // 2-adic valuations 0 .. M-1 (their "classes"; M: a multiple of 2^M).  The
 // classes below come from a search over all windows of a tile (and the
 // natural and the coalesced layout); tests/test_win_layout.py counts the
-// conflicts that are left.  One bit of each class takes the weights 1, 2, 4,
+// conflicts that are left, and tests/test_win_network.py runs the network of
+// win.cuh on these tables.  One bit of each class takes the weights 1, 2, 4,
 // ..; the others follow in the order of their class, each the smallest value
 // of its class above the sum of all before it, which keeps every address
 // unique and the region within a few percent of 2^LOGW.

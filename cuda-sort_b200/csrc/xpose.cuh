@@ -435,7 +435,7 @@ __device__ __forceinline__ void xp_store_striped(typename E::Reg (&v)[1 << LK], 
 }
 
 // Load in natural order straight from memory (the sortedness check, record
-// buffers that are only 4-byte aligned); payloads of gathered types to pay.
+// buffers that are not aligned to the record); payloads of gathered types to pay.
 template <class E, int LK>
 __device__ __forceinline__ void xp_load_natural(typename E::Reg (&v)[1 << LK], const typename E::Mem* src,
                                                 const int t, const int n, int32_t* pay) {
@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB)
 }
 
 // Load, sort and store the arrays of one warp (array of n elements per G-lane
-// team).  Record buffers that are only 4-byte aligned move word by word.
+// team).  Record buffers that are not aligned to the record move in natural order.
 template <class E, int LK, int LG, int IO>
 __device__ __forceinline__ void xp_sort_array(const typename E::Mem* src, typename E::Mem* dst, const int n,
                                               const int t, typename E::Reg* sm, int32_t* pay = nullptr) {

@@ -70,8 +70,8 @@ typedef enum b200s_dtype {
 #define B200S_SORTED_CHECK 2u /* the reference's `Sorted` switch (cusort_v6.hpp:103-128): the
                                  packed path tests each array before sorting and skips the
                                  network when it is already in order (in place: the store
-                                 too); the transposed-network form also tests after every
-                                 stage of span >= 16.  The output is identical either way.
+                                 too); the one-warp tiles of the transposed-network form
+                                 also test after every stage of span >= 16.  The output is identical either way.
                                  The TMA form runs form 0 instead; the cluster and ragged
                                  paths accept the flag and sort in full. */
 #define B200S_PLAN_NO_GRAPH 0x100u /* plan flag: launch the ragged sequence directly
@@ -180,7 +180,9 @@ b200s_status b200s_sort_packed(b200s_dtype dtype, const void* d_in, void* d_out,
  * and, unless B200S_PLAN_NO_GRAPH is set, a CUDA graph of the launch sequence:
  * a call with the previous call's buffers and array count captures and replays
  * it; a call with others, or on a stream that is being captured, launches the
- * sequence directly.  Calls of one plan on different streams are ordered.  Replaces
+ * sequence directly.  Calls of one plan on different streams are ordered, whatever
+ * handles name the streams, but for a sequence that was captured: nothing orders
+ * the replays of the caller's graph against other calls, and the caller has to.  Replaces
  * the reference's partition sort over CSR partitions
  * (SortPartitionsAdaptive_outofplace, cusort.hpp:2309-2352). */
 typedef struct b200s_plan b200s_plan;
@@ -234,7 +236,8 @@ int32_t b200s_plan_plain_launches(const b200s_plan* plan);
  * 48 KB rule to a separate merge sort); longer ones are not written to d_out,
  * and the caller sorts them as the reference's merge path does.
  * Backed by a ragged plan cached per device, element type and stream (one
- * allocation the first time);
+ * allocation the first time), which host threads may share: calls on one
+ * stream take turns;
  * b200s_release_partition_plans frees the cached plans. */
 b200s_status b200s_sort_partitions(b200s_dtype dtype, uint32_t flags, const void* d_in, void* d_out,
                                    const int32_t* d_counters, const int32_t* d_uniform, int32_t nb_parts,
